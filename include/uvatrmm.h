@@ -77,7 +77,10 @@ UVATRMM_API void cblas_dtrmm(CBLAS_LAYOUT layout, CBLAS_SIDE side, CBLAS_UPLO up
 typedef struct uvatrmm_handle_st *uvatrmm_handle_t;
 
 /* Creates a handle bound to the current CUDA device.  A handle owns its
- * workspace and stream setting; use one handle per host thread. */
+ * workspace and stream setting; use one handle per host thread.  The
+ * workspace grows to what the largest call needed and is freed with the
+ * handle.  Device calls may be captured into CUDA graphs; a graph stays valid
+ * as long as the handle, whatever is called on the handle in between. */
 UVATRMM_API int uvatrmm_create(uvatrmm_handle_t *handle);
 UVATRMM_API int uvatrmm_destroy(uvatrmm_handle_t handle);
 /* Stream (a cudaStream_t) for the handle's device work; NULL = legacy default stream. */

@@ -52,12 +52,28 @@ uvatrmm_handle_t resolve(uvatrmm_handle_t h) {
   return tl_default[dev];
 }
 
+bool stream_captures(uvatrmm_handle_t h) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (h->stream && cudaStreamIsCapturing(h->stream, &cap) != cudaSuccess) cudaGetLastError();
+  return cap != cudaStreamCaptureStatusNone;
+}
+
 void *workspace(uvatrmm_handle_t h, int slot, size_t bytes) {
   if (bytes == 0) bytes = 16;
-  if (h->ws_cap[slot] >= bytes) return h->ws[slot];
+  const bool captures = stream_captures(h);
+  if (h->ws_cap[slot] >= bytes) {
+    h->ws_captured[slot] |= captures;
+    return h->ws[slot];
+  }
   if (h->ws[slot]) {
-    cudaStreamSynchronize(h->stream);
-    cudaFree(h->ws[slot]);
+    // A graph may replay on a block that a captured call was given: it stays
+    // until the handle goes.
+    if (h->ws_captured[slot] || captures) {
+      h->ws_kept.push_back(h->ws[slot]);
+    } else {
+      cudaStreamSynchronize(h->stream);
+      cudaFree(h->ws[slot]);
+    }
     h->ws[slot] = nullptr;
     h->ws_cap[slot] = 0;
   }
@@ -69,18 +85,14 @@ void *workspace(uvatrmm_handle_t h, int slot, size_t bytes) {
     return nullptr;
   }
   h->ws_cap[slot] = cap;
+  h->ws_captured[slot] = captures;
   return h->ws[slot];
 }
 
 bool small_scratch(uvatrmm_handle_t h, SmallProduct *p) {
   const size_t need = small_part_bytes(*p);
   if (!need) return true;
-  bool may = true;
-  if (h->ws_cap[3] < need && h->stream) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(h->stream, &cap) != cudaSuccess) cudaGetLastError();
-    may = cap == cudaStreamCaptureStatusNone;
-  }
+  const bool may = h->ws_cap[3] >= need || !stream_captures(h);
   if (may && (p->part = static_cast<double *>(workspace(h, 3, need)))) return true;
   ok();
   p->kc = 0;
@@ -405,6 +417,7 @@ UVATRMM_API int uvatrmm_destroy(uvatrmm_handle_t h) {
   cudaStreamSynchronize(h->stream);
   for (int i = 0; i < uvatrmm_handle_st::kSlots; ++i)
     if (h->ws[i]) cudaFree(h->ws[i]);
+  for (void *p : h->ws_kept) cudaFree(p);
   if (h->dctl) cudaFree(h->dctl);
   if (h->ev0) cudaEventDestroy(h->ev0);
   if (h->ev1) cudaEventDestroy(h->ev1);

@@ -38,6 +38,10 @@ struct uvatrmm_handle_st {
   static constexpr int kSlots = 8;
   void *ws[kSlots] = {};
   size_t ws_cap[kSlots] = {};
+  // Slots whose block was handed out during a stream capture, and such blocks
+  // that were outgrown: kept until the handle goes, as a graph may use them.
+  bool ws_captured[kSlots] = {};
+  std::vector<void *> ws_kept;
   // [0] tile counter, [1] kernel status word, [2], [3] the server's tile
   // counters; the lossless route's OzCtl at kHandleCtlOffset, the scaling's
   // counters at kHandleCountersOffset, its blocks' words at kHandleSlotsOffset.
@@ -73,6 +77,8 @@ uvatrmm_handle_t resolve(uvatrmm_handle_t h);
 
 // Ensures workspace slot `slot` holds at least `bytes`; returns its pointer or nullptr.
 void *workspace(uvatrmm_handle_t h, int slot, size_t bytes);
+// True while the handle's stream is being captured into a graph.
+bool stream_captures(uvatrmm_handle_t h);
 
 // Host <-> device 2-D copy (`width` bytes x `height` lines) for the host
 // entry points, ordered on h->stream.  Host memory from uvatrmm_host_alloc

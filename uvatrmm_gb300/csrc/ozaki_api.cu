@@ -329,9 +329,7 @@ int exact_product(uvatrmm_handle_t h, const OzOperand &L, const OzOperand &R, bo
   for (int k = 0; k < 3; ++k)
     if (h->ws_cap[4 + k] < need[k]) grow += need[k];
   if (grow) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (h->stream && cudaStreamIsCapturing(h->stream, &cap) != cudaSuccess) cudaGetLastError();
-    if (cap != cudaStreamCaptureStatusNone) return UVATRMM_OK;
+    if (stream_captures(h)) return UVATRMM_OK;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b / 2 < grow) {
       cudaGetLastError();
