@@ -86,3 +86,60 @@ def test_replays_survive_a_larger_call_on_the_handle(built, make):
         torch.cuda.synchronize()
         h.close()
         other.close()
+
+
+@pytest.mark.parametrize("make", [lambda: trmm_oop(512, 500), lambda: trmm_oop(1000, 5), lambda: gemm(900, 640, 520)])
+@pytest.mark.parametrize("outgrown", [False, True])
+def test_growing_a_workspace_does_not_end_another_threads_capture(built, make, outgrown):
+    """A call allocates its workspace, and frees the smaller one it had, while
+    another thread captures in CUDA's global mode: both come out right."""
+    import threading
+
+    import torch
+    call, shape_a, shape_b = make()
+    A, B = rand(1, *shape_a), rand(2, *shape_b)
+    m_out = shape_b[1] if call.__qualname__.split(".")[0] != "gemm" else shape_a[1]
+    want = torch.zeros(shape_b[0], m_out, dtype=torch.float64, device="cuda")
+    got, x = torch.zeros_like(want), torch.zeros(1000, device="cuda")
+    st, warm = torch.cuda.Stream(), u.Handle()
+    torch.cuda.synchronize()
+    call(warm, A, B, want)  # (loads the kernels, too)
+    warm.sync()
+    fresh = u.Handle(stream=st)
+    if outgrown:
+        for m, n in ((300, 300), (86, 1)):
+            trmm_oop(m, n)[0](fresh, rand(3, m, m), rand(4, n, m), torch.zeros(n, m, dtype=torch.float64, device="cuda"))
+        fresh.sync()
+    torch.cuda.synchronize()
+    began, called, seen = threading.Event(), threading.Event(), {}
+
+    def capture():
+        try:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=torch.cuda.Stream(), capture_error_mode="global"):
+                x.add_(1)
+                began.set()
+                called.wait(30)
+                x.add_(1)
+            graph.replay()
+            torch.cuda.synchronize()
+            seen["x"] = float(x[0])
+        except Exception as e:  # noqa: BLE001
+            seen["error"] = e
+        finally:
+            began.set()
+
+    t = threading.Thread(target=capture)
+    t.start()
+    began.wait(30)
+    try:
+        call(fresh, A, B, got)
+    finally:
+        called.set()
+        t.join()
+    fresh.sync()
+    torch.cuda.synchronize()
+    assert seen == {"x": 2.0}
+    assert torch.equal(got, want)
+    fresh.close()
+    warm.close()

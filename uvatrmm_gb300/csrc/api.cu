@@ -4,6 +4,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <optional>
 #include <string>
 
 #include "api_internal.h"
@@ -52,6 +53,21 @@ uvatrmm_handle_t resolve(uvatrmm_handle_t h) {
   return tl_default[dev];
 }
 
+namespace {
+
+// cudaMalloc and cudaFree end a capture that another thread has begun in
+// CUDA's global mode, unless the calling thread's own mode allows them.
+struct CaptureModeRelaxed {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  CaptureModeRelaxed() { swap(); }
+  ~CaptureModeRelaxed() { swap(); }
+  void swap() {
+    if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) cudaGetLastError();
+  }
+};
+
+}  // namespace
+
 bool stream_captures(uvatrmm_handle_t h) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (h->stream && cudaStreamIsCapturing(h->stream, &cap) != cudaSuccess) cudaGetLastError();
@@ -65,6 +81,9 @@ void *workspace(uvatrmm_handle_t h, int slot, size_t bytes) {
     h->ws_captured[slot] |= captures;
     return h->ws[slot];
   }
+  // (During a capture of its own stream a call allocates as its capture's mode allows.)
+  std::optional<CaptureModeRelaxed> relaxed;
+  if (!captures) relaxed.emplace();
   if (h->ws[slot]) {
     // A graph may replay on a block that a captured call was given: it stays
     // until the handle goes.
