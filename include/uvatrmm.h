@@ -105,10 +105,15 @@ typedef enum {
                                        the plain FP64 kernels of this handle wait N polls on a barrier
                                        that nothing completes, so they end with UVATRMM_ETIMEOUT at the
                                        next uvatrmm_sync (the context stays usable) */
-  UVATRMM_OPT_OZAKI_ERR_HOST = 11   /* 1: uvatrmm_ozaki_dtrmm_device's relerr_out is measured against
+  UVATRMM_OPT_OZAKI_ERR_HOST = 11,  /* 1: uvatrmm_ozaki_dtrmm_device's relerr_out is measured against
                                        the host FP64 reference (A and the samples copied to the host),
                                        as uvatrmm_ozaki_dtrmm's always is; 0 (default): against the
                                        plain FP64 kernel on the device */
+  UVATRMM_OPT_EXCHANGE_EXPIRY_TEST = 12 /* tests of the failure path only: 0 = off (default); N > 0 makes
+                                       one block of the lossless route's scaling wait N polls for a word
+                                       that nothing writes (calls whose scaling and slicing are one
+                                       launch): the FP64 kernels then compute the call, and the next
+                                       uvatrmm_sync gives UVATRMM_ETIMEOUT */
 } uvatrmm_option;
 typedef enum { UVATRMM_ENGINE_DFMA = 0, UVATRMM_ENGINE_DMMA = 1 } uvatrmm_engine;
 /* Routes of an FP64 call.  On a handle whose engine, tile, schedule and

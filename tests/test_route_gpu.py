@@ -1,0 +1,53 @@
+"""The lossless route of the FP64 calls at its edges: waits that run out, calls
+it declines, handles and options that keep it off or bound it."""
+import numpy as np
+import pytest
+
+import uvatrmm_gb300 as u
+from oracle import oracle as orc
+from tests.helpers import COL, EPS, LEFT, LOWER, NONUNIT, NOTRANS, RIGHT, TRANS, UPPER
+from tests.test_exact_gpu import operands, run
+
+pytestmark = pytest.mark.gpu
+
+
+def oracle_dd(side, uplo, trans, m, n, alpha, A, lda, B, ldb):
+    return orc.dtrmm_dd(COL, side, uplo, trans, NONUNIT, m, n, alpha, A.cpu().numpy().ravel(), lda,
+                        B.cpu().numpy().ravel(), ldb)
+
+
+def assert_fp64_tier(got, want, k):
+    err = np.linalg.norm(got - want) / np.linalg.norm(want)
+    assert err <= 8 * k * EPS, err
+
+
+@pytest.mark.parametrize("side,m,n", [(LEFT, 400, 300), (RIGHT, 129, 512), (LEFT, 512, 700)])
+def test_an_exchange_that_runs_out_leaves_the_call_to_the_fp64_kernels(built, side, m, n):
+    """One block of the one-launch scaling gives up its wait: it has cut no
+    residues, so the call is the FP64 kernels', right and reported as
+    ETIMEOUT; the calls after it take the route again."""
+    h = u.Handle()
+    ka = m if side == LEFT else n
+    try:
+        A0, lda, B0, ldb = operands(side, UPPER, m, n, "normal", pad=1)
+        run(h, side, UPPER, NOTRANS, NONUNIT, m, n, 1.0, A0, lda, B0, ldb, in_place=True)  # other planes
+        A, lda, B, ldb = operands(side, UPPER, m, n, "uniform", pad=1)
+        want = oracle_dd(side, UPPER, NOTRANS, m, n, 1.5, A, lda, B, ldb)
+        for _ in range(2):
+            for in_place in (True, False):
+                h.set_option("exchange_expiry_test", 1000)
+                out = B.clone()
+                if in_place:
+                    h.dtrmm_device(COL, side, UPPER, NOTRANS, NONUNIT, m, n, 1.5, A, lda, out, ldb)
+                else:
+                    h.dtrmm_device_oop(COL, side, UPPER, NOTRANS, NONUNIT, m, n, 1.5, A, lda, B, ldb, out, ldb)
+                with pytest.raises(u.UvatrmmError) as ei:
+                    h.sync()
+                assert ei.value.status == u.ETIMEOUT
+                h.set_option("exchange_expiry_test", 0)
+                assert_fp64_tier(out.cpu().numpy()[:, :m].T, want, ka)
+                one = oracle_dd(side, UPPER, NOTRANS, m, n, 1.0, A, lda, B, ldb)
+                got = run(h, side, UPPER, NOTRANS, NONUNIT, m, n, 1.0, A, lda, B, ldb, in_place)
+                assert np.array_equal(got[:, :m].T, one)
+    finally:
+        h.close()

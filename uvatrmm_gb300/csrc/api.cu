@@ -495,6 +495,10 @@ UVATRMM_API int uvatrmm_set_option(uvatrmm_handle_t h, int option, int value) {
       if (value < 0 || value > (int)kSpinLimit) break;
       h->expiry_test_polls = (uint32_t)value;
       return ok();
+    case UVATRMM_OPT_EXCHANGE_EXPIRY_TEST:
+      if (value < 0 || value > (int)kSpinLimit) break;
+      h->exchange_expiry_polls = (uint32_t)value;
+      return ok();
     case UVATRMM_OPT_AUTOTUNE:
       if (value != 0 && value != 1) break;
       h->autotune = value != 0;

@@ -29,6 +29,7 @@ struct uvatrmm_handle_st {
   bool autotune = true;
   int oz_raster = 0;  // residue-GEMM raster group of single Ozaki calls (0 = default)
   uint32_t expiry_test_polls = 0;  // UVATRMM_OPT_WAIT_EXPIRY_TEST (0 = off)
+  uint32_t exchange_expiry_polls = 0;  // UVATRMM_OPT_EXCHANGE_EXPIRY_TEST (0 = off)
   bool oz_err_host = false;        // UVATRMM_OPT_OZAKI_ERR_HOST
   // Grow-only device workspace slots: 0-2 plain-path and GEMM staging,
   // 3 reductions and the small kernel's partial sums, 4 Ozaki scales, 5 Ozaki residue planes, 6 Ozaki product

@@ -80,8 +80,8 @@ struct OzCtl {
   int span[2];   // widest span
   int nlow[2];   // minus the exponent of the lowest set bit
   int bad;       // a non-finite entry was seen
-  unsigned done;
-  unsigned gen;  // launches of the fused kernel so far
+  unsigned done;  // row tiles (fused kernel: blocks) that have arrived
+  unsigned gen;   // launches of the fused kernel so far
 };
 constexpr OzCtl kOzCtlInit{0, 0, {0, 0}, {kExpNone, kExpNone}, {kExpNone, kExpNone}, 0, 0u, 0u};
 constexpr int kMaxBits = 126;  // what the slicing's digits hold
@@ -150,11 +150,15 @@ int oz_residues(const OzOperand &L, const OzOperand &R, const int *e_row, const 
                 const OzCtl *ctl, int l0, int l1, uint16_t *LR, uint16_t *RR, cudaStream_t st);
 // oz_scales and oz_residues (all moduli) in one launch, for operands whose rows
 // fit the SMs' shared memory; `taken` says whether it was launched.  `slots`:
-// kFusedSlots words, zero at first, used by one launch at a time (with `ctl`).
+// kFusedSlots words, zero at first, used by one launch at a time (with `ctl`;
+// the last one is never written).  Where a block's wait for the others' words
+// runs out, the decision is no, so that the FP64 kernel computes the call, and
+// `status` says so; `expiry_polls` (0: off) makes one block's wait run out
+// after that many polls.
 constexpr int kFusedSlots = 1024;
 int oz_prep_once(const OzOperand &L, const OzOperand &R, const OzScaleBuf &b, const OzPlan &plan, OzCtl *ctl, int *zero,
-                 unsigned long long *slots, uint16_t *LR, uint16_t *RR, int *status, int num_sms, cudaStream_t st,
-                 bool *taken);
+                 unsigned long long *slots, uint16_t *LR, uint16_t *RR, int *status, int num_sms, unsigned expiry_polls,
+                 cudaStream_t st, bool *taken);
 // CRT reassembly of C = alpha * product + beta * C (column-major, ldc) from
 // residue planes res[l][j / 2][i][j % 2] (uint16, plane stride Mp*Np).  Where
 // the route's decision says no, C is copied to `stage` (unless null) instead.

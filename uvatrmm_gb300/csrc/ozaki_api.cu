@@ -190,7 +190,7 @@ int ozaki_device(uvatrmm_handle_t h, int layout, int side, int uplo, int transa,
   int rc = UVATRMM_OK;
   if (G == plan.n_moduli && !h->stage_timing)
     rc = oz_prep_once(L, R, sb, plan, nullptr, nullptr, nullptr, planes, planes + (int64_t)G * plan.Mp * plan.Kp, h->dctl + 1,
-                      h->num_sms, h->stream, &sliced);
+                      h->num_sms, 0, h->stream, &sliced);
   if (rc == UVATRMM_OK && !sliced) rc = oz_scales(L, R, sb, scale_counters(h), nullptr, nullptr, h->stream);
   if (rc != UVATRMM_OK) return fail(rc, "Ozaki scaling failed to launch");
   mark(0);
@@ -345,8 +345,8 @@ int exact_product(uvatrmm_handle_t h, const OzOperand &L, const OzOperand &R, bo
   bool sliced = false;
   int rc = UVATRMM_OK;
   if (panels == 1 && G == plan.n_moduli)
-    rc = oz_prep_once(L, R, sb, plan, ctl, h->dctl, fused_slots(h), planes, planes + G * plan.Mp * plan.Kp, h->dctl + 1, h->num_sms,
-                      h->stream, &sliced);
+    rc = oz_prep_once(L, R, sb, plan, ctl, h->dctl, fused_slots(h), planes, planes + G * plan.Mp * plan.Kp,
+                      h->dctl + 1, h->num_sms, h->exchange_expiry_polls, h->stream, &sliced);
   if (rc == UVATRMM_OK && !sliced) rc = oz_scales(L, R, sb, scale_counters(h), ctl, h->dctl, h->stream);
   if (rc != UVATRMM_OK) return fail(rc, "scaling failed to launch");
   for (int64_t c0 = 0; c0 < (by_cols ? plan.N : plan.M); c0 += w) {

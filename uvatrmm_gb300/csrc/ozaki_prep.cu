@@ -694,12 +694,15 @@ __global__ void __launch_bounds__(256, 3) residue_kernel(const __grid_constant__
 constexpr int FR = 8;    // rows per block
 constexpr int NT = 512;  // threads; 16 warps have an SM's slicing well in flight
 constexpr uint32_t kFusedSpin = 1u << 21;
+constexpr unsigned kLostBlock = 1u << 16;  // OzCtl::done counts blocks below this, blocks whose wait ran out above
+static_assert(kFusedSlots < (int)kLostBlock, "");
 
 struct FusedJob {
   ScaleJob L, R;  // tiles: blocks of FR rows
   ResidueJob rL, rR;
   unsigned long long *slots;  // one word per block
   int *status;
+  unsigned expiry_polls;  // tests: the last block first waits this long for a word that nothing writes
 };
 
 // What a block tells the others: the launch's number, whether its rows hold a
@@ -712,8 +715,9 @@ __device__ __forceinline__ unsigned long long slot_word(unsigned gen, int span, 
 template <bool SPAN>
 __global__ void __launch_bounds__(NT, 1) fused_kernel(const __grid_constant__ FusedJob F) {
   extern __shared__ __align__(16) double rows[];  // [FR][ld], k from kb on
-  __shared__ int red[FR], redn[FR], all[5], dec[2];
+  __shared__ int red[FR], redn[FR], all[6], dec[4];  // (all[5]: a wait of this block ran out)
   __shared__ unsigned gen;  // this launch's number
+  unsigned arrived = 0;
   chain_wait();
   const int nleft = F.L.tiles, nblocks = nleft + F.R.tiles;
   const bool left = (int)blockIdx.x < nleft;
@@ -733,7 +737,7 @@ __global__ void __launch_bounds__(NT, 1) fused_kernel(const __grid_constant__ Fu
     else kb = blk;
   }
   if (tid < FR) red[tid] = redn[tid] = kExpNone;
-  if (SPAN && tid < 5) all[tid] = tid < 4 ? kExpNone : 0;
+  if (SPAN && tid < 6) all[tid] = tid < 4 ? kExpNone : 0;
   if (SPAN && tid == 0) gen = *(volatile unsigned *)&S.ctl->gen + 1;
   {
     // All of the rows' loads are in flight at once; a warp reads along k, or
@@ -787,15 +791,18 @@ __global__ void __launch_bounds__(NT, 1) fused_kernel(const __grid_constant__ Fu
     }
     // Every block reads every block's word.
     int span[2] = {kExpNone, kExpNone}, low[2] = {kExpNone, kExpNone}, bad = 0;
-    for (int i = tid; i < nblocks; i += NT) {
+    bool lost = false;
+    auto word = [&](int i, uint32_t polls) {
       unsigned long long v;
       uint32_t it = 0;
       do v = *(volatile unsigned long long *)(F.slots + i);
-      while ((unsigned)(v >> 32) != gen && ++it < kFusedSpin);
-      if (it == kFusedSpin) {
-        record_error(F.status, KERR_WAIT_TIMEOUT);
-        v = 0x80000000u;
-      }
+      while ((unsigned)(v >> 32) != gen && ++it < polls);
+      lost = lost || it >= polls;
+      return v;
+    };
+    if (F.expiry_polls && (int)blockIdx.x == nblocks - 1 && tid == 0) word(kFusedSlots - 1, F.expiry_polls);
+    for (int i = tid; i < nblocks; i += NT) {
+      const unsigned long long v = word(i, kFusedSpin);
       const int s = (int)(v & 0xFFFu), side = i >= nleft;
       if (s) {
         span[side] = max(span[side], s);
@@ -808,28 +815,31 @@ __global__ void __launch_bounds__(NT, 1) fused_kernel(const __grid_constant__ Fu
     if (low[0] != kExpNone) atomicMax(&all[2], low[0]);
     if (low[1] != kExpNone) atomicMax(&all[3], low[1]);
     if (bad) atomicMax(&all[4], 1);
+    if (lost) {
+      record_error(F.status, KERR_WAIT_TIMEOUT);
+      atomicMax(&all[5], 1);
+    }
     __syncthreads();
+    // The last block to get here publishes (when its last warp, which has the
+    // least to cut, is done: nothing waits for this atomic): the launch's
+    // number, as every block has read the one before, and the decision, a no
+    // where any block's wait ran out, as that block has cut no residues.
+    if (tid == NT - 32) arrived = atomicAdd(&S.ctl->done, all[5] ? kLostBlock + 1u : 1u);
     if (w == 0) {
       int go, n, b0, b1;
       decide(all[0], all[1], all[2], all[3], all[4] != 0, S.klog, go, n, b0, b1);
       if (ln == 0) {
-        dec[0] = go ? n : 0;
-        dec[1] = left ? b0 : b1;
-        if (blockIdx.x == 0) {
-          S.ctl->go = go;
-          S.ctl->n = n;
-          S.ctl->bits[0] = b0;
-          S.ctl->bits[1] = b1;
-          S.ctl->gen = gen;  // (all blocks have read it: their words are here)
-          if (S.zero) *S.zero = 0;
-        }
+        dec[0] = go && !all[5] ? n : 0;
+        dec[1] = n;
+        dec[2] = b0;
+        dec[3] = b1;
       }
     }
     __syncthreads();
   }
   const int l1 = __reduce_max_sync(0xffffffffu, SPAN ? dec[0] : J.l1);
-  const int bits = __reduce_max_sync(0xffffffffu, SPAN ? dec[1] : J.bits);
-  if (l1 == 0) return;
+  const int bits = __reduce_max_sync(0xffffffffu, SPAN ? dec[left ? 2 : 3] : J.bits);
+  if (l1 == 0) ke = kb;
   const int64_t plane = J.Pp * J.Kp;
   const int r = tid / (NT / 4);
   int ep[2] = {red[r], red[r + FR / 2]};
@@ -847,6 +857,16 @@ __global__ void __launch_bounds__(NT, 1) fused_kernel(const __grid_constant__ Fu
       v[h][3] = c.y;
     }
     slice_rows(v, bits, ep, 0, l1, J.R + (p0 + r) * J.Kp + k, plane, (FR / 2) * J.Kp);
+  }
+  if (SPAN && tid == NT - 32 && (arrived & (kLostBlock - 1)) == (unsigned)nblocks - 1) {
+    const bool whole = arrived < kLostBlock;
+    S.ctl->go = dec[0] != 0 && whole;
+    S.ctl->n = dec[1];
+    S.ctl->bits[0] = dec[2];
+    S.ctl->bits[1] = dec[3];
+    S.ctl->gen = gen;
+    S.ctl->done = 0u;
+    if (S.zero) *S.zero = 0;
   }
 }
 
@@ -1445,8 +1465,8 @@ int oz_residues(const OzOperand &L, const OzOperand &R, const int *e_row, const 
 }
 
 int oz_prep_once(const OzOperand &L, const OzOperand &R, const OzScaleBuf &b, const OzPlan &plan, OzCtl *ctl, int *zero,
-                 unsigned long long *slots, uint16_t *LR, uint16_t *RR, int *status, int num_sms, cudaStream_t st,
-                 bool *taken) {
+                 unsigned long long *slots, uint16_t *LR, uint16_t *RR, int *status, int num_sms, unsigned expiry_polls,
+                 cudaStream_t st, bool *taken) {
   *taken = false;
   // A row's line is 16-byte aligned, and eight rows' lines start in different
   // banks.
@@ -1457,7 +1477,7 @@ int oz_prep_once(const OzOperand &L, const OzOperand &R, const OzScaleBuf &b, co
   // 47.3 / 45.6, 1000 x 200 45.0 / 40.4 (wide entries 68 / 61); emulated tier,
   // 20 moduli, 1000 x 200 44.0 / 46.7, 1150 x 60 52.4 / 48.1.
   constexpr int kMaxK = 1024;
-  if (blocks > std::min(num_sms, kFusedSlots) || plan.Kp > (ctl ? 512 : kMaxK)) return UVATRMM_OK;
+  if (blocks > std::min(num_sms, kFusedSlots - 1) || plan.Kp > (ctl ? 512 : kMaxK)) return UVATRMM_OK;
   FusedJob f;
   f.L = scale_job(L, 0, b, ctl, L.K);
   f.R = scale_job(R, 1, b, ctl, R.K);
@@ -1468,6 +1488,7 @@ int oz_prep_once(const OzOperand &L, const OzOperand &R, const OzScaleBuf &b, co
   f.rR = residue_job(R, 1, b.e_col, plan, ctl, 0, plan.n_moduli, RR);
   f.slots = slots;
   f.status = status;
+  f.expiry_polls = expiry_polls;
   auto kernel = ctl ? fused_kernel<true> : fused_kernel<false>;
   if (smem > (48 << 10) && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 FR * (kMaxK + 2) * (int)sizeof(double)) != cudaSuccess) {
