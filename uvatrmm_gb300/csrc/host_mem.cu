@@ -15,9 +15,12 @@
 // staging chunk are moved by a kernel that reads or writes them where they
 // lie: the GPU shares the host's page tables over NVLink-C2C and moves 200
 // GB/s in and 170 GB/s out (8 MB: 52 us), where one CPU core packs 10 GB/s.
-// Larger ones, whose pages may have aged, are packed into two staging buffers
-// of the above kind by several CPU threads, each chunk's DMA overlapping the
-// packing of the next (host_copy2d).
+// Every page of them is touched on the host first (host_touch.h).  Larger ones
+// are packed into two staging buffers of the above kind by several CPU threads,
+// each chunk's DMA overlapping the packing of the next (host_copy2d).  (Just
+// above the default chunk the packing is the slower of the two, whole calls of
+// m = n = 5800, 257 MiB: 11.2 against 6.9 ms; 8192: 21.6 / 14.7, warm.  A larger
+// UVATRMM_OPT_HOST_STAGE_KB moves the line.)
 #include <sys/mman.h>
 #include <unistd.h>
 
@@ -32,6 +35,7 @@
 #include <vector>
 
 #include "api_internal.h"
+#include "host_touch.h"
 
 namespace uvt {
 namespace {
@@ -119,25 +123,17 @@ __global__ void __launch_bounds__(256) host_move_kernel(double *dst, int64_t dpi
   }
 }
 
-// Touches the host lines' ends, so that a bad pointer faults here and not on
-// the GPU, and, with `write`, every page of them, so that the GPU does not
-// wait for the kernel to map a new buffer's pages one by one.
-void touch_lines(const void *host, size_t pitch, size_t width, size_t lines, bool write) {
-  const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-  volatile const char *p = static_cast<const char *>(host);
-  (void)p[0];
-  (void)p[pitch * (lines - 1) + width - 1];
-  if (!write) return;
-  uintptr_t last = 0;
-  for (size_t l = 0; l < lines; ++l) {
-    volatile char *b = static_cast<char *>(const_cast<void *>(host)) + l * pitch;
-    for (size_t at = 0; at < width; at += std::min(page, std::max<size_t>(1, width - 1 - at))) {
-      const uintptr_t pg = reinterpret_cast<uintptr_t>(b + at) / page;
-      if (pg != last) b[at] = b[at];
-      last = pg;
-      if (at + 1 >= width) break;
-    }
-  }
+// Touches every page of the host lines (of the triangle, see line_part), so
+// that a bad pointer or a hole in the operand faults here and not on the GPU,
+// and, with `write`, so that the GPU does not wait for the kernel to map a new
+// buffer's pages one by one.
+void touch_lines(const void *host, size_t pitch, size_t width, size_t lines, int tri, bool write) {
+  for_each_page(reinterpret_cast<uintptr_t>(host), pitch, width, lines, tri, (size_t)sysconf(_SC_PAGESIZE),
+                [&](uintptr_t a) {
+                  volatile char *b = reinterpret_cast<volatile char *>(a);
+                  const char c = *b;
+                  if (write) *b = c;
+                });
 }
 
 // Moves the lines by a kernel, where it can: sizes in bytes.
@@ -151,7 +147,7 @@ bool move_by_kernel(uvatrmm_handle_t h, void *dst, size_t dpitch, const void *sr
     dpitch = spitch = width;
     lines = 1;
   }
-  touch_lines(h2d ? src : dst, h2d ? spitch : dpitch, width, lines, !h2d);
+  touch_lines(h2d ? src : dst, h2d ? spitch : dpitch, width, lines, tri, !h2d);
   const uint32_t total = (uint32_t)(width / 8 * lines);
   const unsigned grid = std::min<unsigned>((total + 1023) / 1024, (unsigned)h->num_sms * 8);
   host_move_kernel<<<grid, 256, 0, h->stream>>>(static_cast<double *>(dst), (int64_t)(dpitch / 8),
