@@ -93,7 +93,8 @@ typedef enum {
   UVATRMM_OPT_SCHEDULE = 2, /* UVATRMM_SCHED_*    tile-to-SM assignment */
   UVATRMM_OPT_SHAPE = 3,    /* UVATRMM_SHAPE_*    diagonal tile geometry */
   UVATRMM_OPT_TILE = 4,     /* 0 = automatic, 64 or 128: output tile edge */
-  UVATRMM_OPT_OZAKI_SCRATCH_MB = 5, /* Ozaki residue-plane budget per pass, MiB (default 49152) */
+  UVATRMM_OPT_OZAKI_SCRATCH_MB = 5, /* Ozaki residue-plane budget per pass, MiB (default 49152); also the
+                                       most scratch a call of the lossless route takes */
   UVATRMM_OPT_STAGE_TIMING = 6,     /* 1: time the stages of each Ozaki call (uvatrmm_stage_times) */
   UVATRMM_OPT_AUTOTUNE = 7,         /* 1 (default): measure untuned shape buckets; 0: defaults only */
   UVATRMM_OPT_OZAKI_RASTER = 8,     /* Ozaki residue GEMM of single calls: major tiles per raster
@@ -125,8 +126,9 @@ typedef enum { UVATRMM_ENGINE_DFMA = 0, UVATRMM_ENGINE_DMMA = 1 } uvatrmm_engine
  * FP64 engines'.  The device decides per call whether the operands allow it
  * (finite entries, about 120 bits between the largest entry and the lowest
  * set bit of a row of op(A) or column of B, no subnormal results);
- * otherwise, or without room for its scratch (at most 16 GiB and half of the
- * free memory), the FP64 tile kernel computes the call. */
+ * otherwise, or without room for its scratch (at most 16 GiB, half of the
+ * free memory and UVATRMM_OPT_OZAKI_SCRATCH_MB), the FP64 kernels compute the
+ * call.  The scratch stays with the handle for its next calls. */
 /* DYNAMIC: persistent CTAs pull tiles from a counter, in bands of 1024
  * columns of the non-triangular operand, longest row tiles first in a band.
  * REG / BALANCED: the reference's row mappings (map_regular / map_balanced)

@@ -51,3 +51,31 @@ def test_an_exchange_that_runs_out_leaves_the_call_to_the_fp64_kernels(built, si
                 assert np.array_equal(got[:, :m].T, one)
     finally:
         h.close()
+
+
+@pytest.mark.parametrize("side,m,n", [(LEFT, 400, 400), (LEFT, 1000, 1000), (RIGHT, 900, 1500), (LEFT, 300, 5000)])
+def test_the_scratch_option_bounds_the_route(built, side, m, n):
+    """With 64 MiB a call goes in panels and passes that fit, in place and out
+    of place, with the same results; the handle takes no more than that."""
+    import torch
+    h, warm = u.Handle(), u.Handle()
+    try:
+        h.set_option("ozaki_scratch_mb", 64)
+        A, lda, B, ldb = operands(side, LOWER, m, n, "wide")
+        want = run(warm, side, LOWER, TRANS, NONUNIT, m, n, 1.0, A, lda, B, ldb, in_place=False)
+        one = oracle_dd(side, LOWER, TRANS, m, n, 1.0, A, lda, B, ldb) if m * n <= 200000 else None
+        out = B.clone()
+        h.sync()
+        torch.cuda.synchronize()
+        free, _ = torch.cuda.mem_get_info()
+        h.dtrmm_device_oop(COL, side, LOWER, TRANS, NONUNIT, m, n, 1.0, A, lda, B, ldb, out, ldb)
+        h.sync()
+        # (The scales' few hundred kilobytes, and 2 MiB steps of three blocks.)
+        assert free - torch.cuda.mem_get_info()[0] <= (64 + 16) << 20
+        assert np.array_equal(out.cpu().numpy(), want)
+        assert one is None or np.array_equal(want[:, :m].T, one)
+        got = run(h, side, LOWER, TRANS, NONUNIT, m, n, 1.0, A, lda, B, ldb, in_place=True)
+        assert np.array_equal(got, want)
+    finally:
+        h.close()
+        warm.close()

@@ -244,9 +244,13 @@ int ozaki_device(uvatrmm_handle_t h, int layout, int side, int uplo, int transa,
   return ok();
 }
 
-// The lossless route (see OzCtl).  Scratch: at most kExactBytes, split between
-// the product residues of a panel of the minor dimension (the one without
-// the triangle) and the residue planes of a pass over the moduli.
+// The lossless route (see OzCtl).  Scratch: at most kExactBytes and the
+// handle's UVATRMM_OPT_OZAKI_SCRATCH_MB, split between the product residues of
+// a panel of the minor dimension (the one without the triangle) and the
+// residue planes of a pass over the moduli.  Down to the option's least value
+// the panels and passes are faster than the tile kernel wherever they fit (us,
+// 64 MiB / tile kernel: 1000 x 1000 146 / 2010, 2000 x 2000 1610 / 7050, 2700 x
+// 2700 8227 / 16952, 300 x 50000 2054 / 4105).
 namespace {
 constexpr int64_t kExactBytes = 16ll << 30;
 }
@@ -315,12 +319,13 @@ int exact_product(uvatrmm_handle_t h, const OzOperand &L, const OzOperand &R, bo
   // Panel width w of the minor dimension and moduli per pass G.
   const bool by_cols = tri_left;  // minor dimension: columns of Rgt, else rows of Lft
   const int64_t major = by_cols ? plan.Mp : plan.Np, minor = by_cols ? plan.Np : plan.Mp;
+  const int64_t limit = std::min(kExactBytes, h->ozaki_scratch_mb << 20);
   const int64_t per_res = 2 * oz_res_planes(kCrtModuli) * major * kOzBlock;  // product residues of 256 minor lines
-  int64_t w = std::min(minor, std::max<int64_t>(1, kExactBytes / 2 / per_res) * kOzBlock);
+  int64_t w = std::min(minor, std::max<int64_t>(1, limit / 2 / per_res) * kOzBlock);
   const int64_t panels = (minor + w - 1) / w;
   w = round_up((minor + panels - 1) / panels, kOzBlock);
   const int64_t res_bytes = per_res * (w / kOzBlock), per_mod = (major + w) * plan.Kp * 2;
-  const int64_t G = std::min<int64_t>(kCrtModuli, (kExactBytes - res_bytes) / per_mod);
+  const int64_t G = std::min<int64_t>(kCrtModuli, (limit - res_bytes) / per_mod);
   if (G < 1) return UVATRMM_OK;
   const size_t need[3] = {oz_scale_bytes(plan.Mp, plan.Np, plan.K), (size_t)(G * per_mod), (size_t)res_bytes};
   // Scratch that is not there yet is taken only outside a stream capture,
