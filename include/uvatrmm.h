@@ -294,8 +294,9 @@ typedef struct {
 
 typedef struct uvatrmm_group_st *uvatrmm_group_t;
 /* Plans the batch: checks every problem, picks its tile shape (autotuner),
- * sizes one workspace arena (Ozaki problems are processed in waves that fit
- * UVATRMM_OPT_OZAKI_SCRATCH_MB), uploads the descriptors and captures the
+ * sizes one workspace arena (Ozaki problems, and FP64 problems on the lossless
+ * route, are processed in waves that fit UVATRMM_OPT_OZAKI_SCRATCH_MB; an FP64
+ * problem that does not fit runs on the tile kernel), uploads the descriptors and captures the
  * whole batch into a CUDA graph on the handle's stream.  The problems'
  * buffers must stay valid while the group lives; every run recomputes each
  * problem from the current contents of its buffers. */

@@ -79,3 +79,36 @@ def test_the_scratch_option_bounds_the_route(built, side, m, n):
     finally:
         h.close()
         warm.close()
+
+
+def test_a_groups_waves_fit_the_scratch_option(built):
+    """FP64 problems join waves that fit the option; one that does not fit by
+    itself (900 x 1500) runs on the tile kernel."""
+    import torch
+    h = u.Handle()
+    try:
+        h.set_option("ozaki_scratch_mb", 64)
+        probs, staged = [], 0
+        for i, (side, m, n) in enumerate([(LEFT, 400, 400), (RIGHT, 300, 450), (LEFT, 900, 1500), (RIGHT, 333, 512)]):
+            A, lda, B, ldb = operands(side, UPPER, m, n, "uniform")
+            probs.append(dict(layout=COL, side=side, uplo=UPPER, transa=NOTRANS, diag=NONUNIT, m=m, n=n, alpha=1.0, A=A,
+                              lda=lda, B=B.clone(), B0=B, ldb=ldb, tier=u.TIER_FP64, moduli=0))
+            staged += 8 * (m + 15) // 16 * 16 * n + 8 * (lda + 15) // 16 * 16 * lda
+        torch.cuda.synchronize()
+        g = u.Group(h, probs)
+        st = g.stats()
+        assert st["arena_bytes"] <= (64 << 20) + staged + (1 << 20)
+        assert st["ozaki_waves"] == 3
+        g.run()
+        h.sync()
+        for i, p in enumerate(probs):
+            m, n = p["m"], p["n"]
+            want = oracle_dd(p["side"], UPPER, NOTRANS, m, n, 1.0, p["A"], p["lda"], p["B0"], p["ldb"])
+            got = p["B"].cpu().numpy()[:, :m].T
+            if i == 2:
+                assert_fp64_tier(got, want, m)
+            else:
+                assert np.array_equal(got, want)
+        g.close()
+    finally:
+        h.close()

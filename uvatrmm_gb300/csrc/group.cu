@@ -83,6 +83,7 @@ struct OzItem {
 
 // Device memory a group's waves take at most once FP64 problems are in them.
 constexpr size_t kExactWaveBytes = size_t(16) << 30;
+size_t exact_wave_bytes(uvatrmm_handle_t h) { return std::min((size_t)h->ozaki_scratch_mb << 20, kExactWaveBytes); }
 
 // One staging copy of the FP64 problems (see stage_wave_kernel).
 struct CopyJob {
@@ -236,7 +237,7 @@ int build(uvatrmm_group_t g, const uvatrmm_trmm_problem *probs, int count, bool 
         x.plan.bits = 0;
         x.raster = 0;
         size_item(x);
-        if (x.bytes <= kExactWaveBytes) {
+        if (x.bytes <= exact_wave_bytes(h)) {
           it.exact = x.ctl = n_exact++;
           it.small = small_behind_exact(t.m, t.n, ka, t.side == CblasLeft);
           oz.push_back(x);
@@ -291,8 +292,7 @@ int build(uvatrmm_group_t g, const uvatrmm_trmm_problem *probs, int count, bool 
   // Waves: greedy packing under the scratch budget, longest K first (the
   // residue GEMM's tiles go out in this order).
   std::stable_sort(oz.begin(), oz.end(), [](const OzItem &x, const OzItem &y) { return x.plan.K > y.plan.K; });
-  size_t budget = (size_t)h->ozaki_scratch_mb << 20;
-  if (n_exact) budget = std::min(budget, kExactWaveBytes);
+  const size_t budget = n_exact ? exact_wave_bytes(h) : (size_t)h->ozaki_scratch_mb << 20;
   std::vector<std::vector<int>> waves;
   size_t wave_bytes = 0, max_wave = 0;
   for (int i = 0; i < (int)oz.size(); ++i) {
