@@ -97,10 +97,11 @@ def test_a_groups_waves_fit_the_scratch_option(built):
         torch.cuda.synchronize()
         g = u.Group(h, probs)
         st = g.stats()
-        assert st["arena_bytes"] <= (64 << 20) + staged + (1 << 20)
-        assert st["ozaki_waves"] == 3
         g.run()
         h.sync()
+        g.close()
+        assert st["arena_bytes"] <= (64 << 20) + staged + (1 << 20)
+        assert st["ozaki_waves"] == 3
         for i, p in enumerate(probs):
             m, n = p["m"], p["n"]
             want = oracle_dd(p["side"], UPPER, NOTRANS, m, n, 1.0, p["A"], p["lda"], p["B0"], p["ldb"])
@@ -109,6 +110,34 @@ def test_a_groups_waves_fit_the_scratch_option(built):
                 assert_fp64_tier(got, want, m)
             else:
                 assert np.array_equal(got, want)
-        g.close()
     finally:
         h.close()
+
+
+@pytest.mark.parametrize("option", [("schedule", u.SCHED_REG), ("shape", u.SHAPE_BOXES), ("tile", 64)])
+def test_a_pinned_handles_gemm_stage_and_product_stay_on_the_tile_kernel(built, option):
+    """A handle whose schedule, shape or tile was set keeps its GEMMs, stages
+    and products on the FP64 tile kernel: bit by bit those of a handle whose
+    engine was."""
+    import torch
+    h, pinned = u.Handle(**dict([option])), u.Handle(engine=u.ENGINE_DFMA)
+    pinned.set_option(*option)
+    n, w, b, hr = 900, 700, 300, 500
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    A, B = (torch.rand(n, n, dtype=torch.float64, device="cuda", generator=gen) * 2 - 1 for _ in range(2))
+    torch.cuda.synchronize()
+    out = []
+    try:
+        for hh in (h, pinned):
+            C = [torch.zeros(n, n, dtype=torch.float64, device="cuda") for _ in range(3)]
+            torch.cuda.synchronize()
+            hh.dgemm_device(COL, NOTRANS, TRANS, n, n, n, -0.5, A, n, B, n, 0.0, C[0], n)
+            hh.stage(n, w, b, hr, A[b:], n, B, n, C[1], n)
+            hh.product(n, u.SCHED_DYNAMIC, u.SHAPE_TRAPEZOID, A, B, C[2])
+            hh.sync()
+            out.append(C)
+        for x, y in zip(*out):
+            assert bool(x.any()) and torch.equal(x, y)
+    finally:
+        h.close()
+        pinned.close()

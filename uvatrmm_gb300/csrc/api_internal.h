@@ -193,10 +193,11 @@ Route pick_route(int64_t M, int64_t N, int64_t K, bool tri, bool tri_left, bool 
 // Behind the lossless route of a TRMM: the small kernel instead of the tile
 // kernel (the same bits) where it is faster.
 bool small_behind_exact(int64_t M, int64_t N, int64_t K, bool tri_left);
-// True when no option pins the handle's FP64 calls to the tile kernel.
+// True when no option pins the handle's FP64 calls to the tile kernel, nor
+// the schedule and shape of this call.
 inline bool route_free(uvatrmm_handle_t h, int schedule, int shape) {
-  return !h->engine_set && !h->tile && !h->expiry_test_polls && schedule == UVATRMM_SCHED_DYNAMIC &&
-         shape == UVATRMM_SHAPE_TRAPEZOID;
+  return !h->engine_set && !h->tile && !h->expiry_test_polls && h->schedule == UVATRMM_SCHED_DYNAMIC &&
+         h->shape == UVATRMM_SHAPE_TRAPEZOID && schedule == UVATRMM_SCHED_DYNAMIC && shape == UVATRMM_SHAPE_TRAPEZOID;
 }
 // Enqueues C := alpha * Lft * Rgt + beta * C by the lossless route and gives
 // the decision word by which the FP64 tile kernel and its staging copies
