@@ -141,3 +141,25 @@ def test_a_pinned_handles_gemm_stage_and_product_stay_on_the_tile_kernel(built, 
     finally:
         h.close()
         pinned.close()
+
+
+@pytest.mark.parametrize("n", [270, 1000, 4096])
+def test_a_products_time_holds_no_allocation(built, n):
+    """uvatrmm_product's seconds on a new handle, whose workspace it takes, are
+    those of its next products (within a factor of two; the allocations take
+    0.2 ms and more)."""
+    import torch
+    A, B = (torch.rand(n, n, dtype=torch.float64, device="cuda") for _ in range(2))
+    C = torch.zeros(n, n, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    warm = u.Handle()
+    for _ in range(3):  # (loads the kernels)
+        warm.product(n, u.SCHED_DYNAMIC, u.SHAPE_TRAPEZOID, A, B, C)
+    first, later = [], []
+    for _ in range(5):
+        h = u.Handle()
+        first.append(h.product(n, u.SCHED_DYNAMIC, u.SHAPE_TRAPEZOID, A, B, C))
+        later += [h.product(n, u.SCHED_DYNAMIC, u.SHAPE_TRAPEZOID, A, B, C) for _ in range(3)]
+        h.close()
+    warm.close()
+    assert np.median(first) <= 2 * np.median(later), (first, later)

@@ -263,7 +263,7 @@ cudaError_t stage_copy(uvatrmm_handle_t h, double *dst, int64_t ldd, const doubl
 // dC receives the result (may equal dB only when `in_place`).
 int device_trmm(uvatrmm_handle_t h, int layout, int side, int uplo, int transa, int diag, int64_t m, int64_t n,
                 double alpha, const double *dA, int64_t lda, const double *dB, int64_t ldb, double *dC,
-                int64_t ldc, bool in_place, int schedule, int shape, double beta, bool plain) {
+                int64_t ldc, bool in_place, int schedule, int shape, double beta, bool plain, cudaEvent_t begin) {
   if (int bad = check_args(layout, side, uplo, transa, diag, m, n, lda, ldb))
     return fail(UVATRMM_EINVAL, "parameter " + std::to_string(bad) + " had an illegal value");
   if (!in_place) {
@@ -286,12 +286,15 @@ int device_trmm(uvatrmm_handle_t h, int layout, int side, int uplo, int transa, 
       const int64_t lb = round_up(t.m, 16);
       double *w = static_cast<double *>(workspace(h, 1, (size_t)lb * t.n * 8));
       if (!w) return tl_status;
+      if (begin) cudaEventRecord(begin, h->stream);
       cudaError_t e = stage_copy(h, w, lb, dB, ldb, t.m, t.n, nullptr);
       if (e != cudaSuccess) return cuda_fail(e, "staging B");
       const SmallProduct q = small_trmm(t, dA, lda, w, lb, dC, ldc, beta);
       sp.X = q.X;
       sp.k_stride = q.k_stride;
       sp.v_stride = q.v_stride;
+    } else if (begin) {
+      cudaEventRecord(begin, h->stream);
     }
     const int rc = launch_small(sp, in_place && !copy, h->stream);
     return rc == UVATRMM_OK ? ok() : fail(rc, "kernel launch failed");
@@ -309,6 +312,14 @@ int device_trmm(uvatrmm_handle_t h, int layout, int side, int uplo, int transa, 
     lb = round_up(t.m, 16);
     B = static_cast<double *>(workspace(h, 1, (size_t)lb * t.n * 8));
     if (!B) return tl_status;
+  }
+  if (begin) {
+    if (route == Route::kExact) {
+      exact_reserve(h, t.m, t.n, ka, t.side == CblasLeft);
+      SmallProduct behind = small_trmm(t, A, la, B, lb, dC, ldc, beta);
+      if (small_behind_exact(t.m, t.n, ka, t.side == CblasLeft)) small_scratch(h, &behind);
+    }
+    cudaEventRecord(begin, h->stream);
   }
   const OzCtl *gate = nullptr;
   if (route == Route::kExact)
@@ -575,10 +586,9 @@ UVATRMM_API int uvatrmm_product(uvatrmm_handle_t h, int64_t n, int schedule, int
   if (schedule < UVATRMM_SCHED_DYNAMIC || schedule > UVATRMM_SCHED_BALANCED)
     return fail(UVATRMM_EINVAL, "unknown schedule");
   if (shape != UVATRMM_SHAPE_TRAPEZOID && shape != UVATRMM_SHAPE_BOXES) return fail(UVATRMM_EINVAL, "unknown shape");
-  cudaEventRecord(h->ev0, h->stream);
   // Row-major C = tril(A) * B, as UVaTRMM/src/mm_triangular.c:319-410 computes it.
   int rc = device_trmm(h, CblasRowMajor, CblasLeft, CblasLower, CblasNoTrans, CblasNonUnit, n, n, 1.0, dA, n, dB,
-                       n, dC, n, false, schedule, shape);
+                       n, dC, n, false, schedule, shape, 0.0, false, h->ev0);
   if (rc != UVATRMM_OK) return rc;
   cudaEventRecord(h->ev1, h->stream);
   rc = collect_status(h);

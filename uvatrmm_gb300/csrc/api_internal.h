@@ -125,10 +125,12 @@ Trmm normalise(int layout, int side, int uplo, int transa, int diag, int64_t m, 
 
 // FP64 TRMM on device buffers (stages misaligned operands, and B when in
 // place, through workspace slots 0 and 1).  `plain`: on the tile kernel even
-// where the lossless route would be taken.
+// where the lossless route would be taken.  `begin` (may be null) is recorded
+// once the workspace is there, ahead of the work.
 int device_trmm(uvatrmm_handle_t h, int layout, int side, int uplo, int transa, int diag, int64_t m, int64_t n,
                 double alpha, const double *dA, int64_t lda, const double *dB, int64_t ldb, double *dC,
-                int64_t ldc, bool in_place, int schedule, int shape, double beta = 0.0, bool plain = false);
+                int64_t ldc, bool in_place, int schedule, int shape, double beta = 0.0, bool plain = false,
+                cudaEvent_t begin = nullptr);
 
 // A small product for trmm_small.cu: out[r, v] = alpha * sum_k T[r, k] X[k, v]
 // + beta * out[r, v] with T R x K (triangular, R = K, or dense).
@@ -208,6 +210,8 @@ inline bool route_free(uvatrmm_handle_t h, int schedule, int shape) {
 int exact_product(uvatrmm_handle_t h, const OzOperand &L, const OzOperand &R, bool tri_none, bool tri_left,
                   bool tri_lower, double alpha, double beta, double *C, int64_t ldc, const OzCtl **gate,
                   double *stage = nullptr, int64_t lds = 0);
+// Takes the route's scratch for such a product ahead of the call.
+void exact_reserve(uvatrmm_handle_t h, int64_t M, int64_t N, int64_t K, bool by_cols);
 // Copies a column-major rows x cols block; with `gate`, only where the
 // lossless route did not compute the result.
 cudaError_t stage_copy(uvatrmm_handle_t h, double *dst, int64_t ldd, const double *src, int64_t lds, int64_t rows,

@@ -303,53 +303,88 @@ bool small_behind_exact(int64_t M, int64_t N, int64_t K, bool tri_left) {
   return small_us(K, tri_left ? N : M, K, true) < tile_us(M, N, K, true);
 }
 
-int exact_product(uvatrmm_handle_t h, const OzOperand &L, const OzOperand &R, bool tri_none, bool tri_left,
-                  bool tri_lower, double alpha, double beta, double *C, int64_t ldc, const OzCtl **gate, double *stage,
-                  int64_t lds) {
-  *gate = nullptr;
+namespace {
+
+// The route's panels and passes for an M x N x K product, and their scratch.
+struct ExactPlan {
   OzPlan plan;
-  plan.M = L.P;
-  plan.N = R.P;
-  plan.K = L.K;
+  int64_t w, panels, G, per_mod;  // panel width of the minor dimension, moduli per pass, bytes of planes per modulus
+  size_t need[3];                 // workspace slots 4 to 6: scales, residue planes, product residues
+};
+
+// False where no panel and pass fits the limit.  by_cols: the minor dimension
+// is the columns of Rgt, else the rows of Lft.
+bool exact_plan(uvatrmm_handle_t h, int64_t M, int64_t N, int64_t K, bool by_cols, ExactPlan *p) {
+  OzPlan &plan = p->plan;
+  plan.M = M;
+  plan.N = N;
+  plan.K = K;
   plan.n_moduli = kCrtModuli;
   plan.bits = 0;
   plan.Mp = oz_pad_rows(plan.M);
   plan.Np = oz_pad_cols(plan.N);
   plan.Kp = round_up(plan.K, 64);
-  // Panel width w of the minor dimension and moduli per pass G.
-  const bool by_cols = tri_left;  // minor dimension: columns of Rgt, else rows of Lft
   const int64_t major = by_cols ? plan.Mp : plan.Np, minor = by_cols ? plan.Np : plan.Mp;
   const int64_t limit = std::min(kExactBytes, h->ozaki_scratch_mb << 20);
   const int64_t per_res = 2 * oz_res_planes(kCrtModuli) * major * kOzBlock;  // product residues of 256 minor lines
-  int64_t w = std::min(minor, std::max<int64_t>(1, limit / 2 / per_res) * kOzBlock);
-  const int64_t panels = (minor + w - 1) / w;
-  w = round_up((minor + panels - 1) / panels, kOzBlock);
-  const int64_t res_bytes = per_res * (w / kOzBlock), per_mod = (major + w) * plan.Kp * 2;
-  const int64_t G = std::min<int64_t>(kCrtModuli, (limit - res_bytes) / per_mod);
-  if (G < 1) return UVATRMM_OK;
-  const size_t need[3] = {oz_scale_bytes(plan.Mp, plan.Np, plan.K), (size_t)(G * per_mod), (size_t)res_bytes};
-  // Scratch that is not there yet is taken only outside a stream capture,
-  // and only where it leaves as much memory free as it takes.
+  const int64_t w = std::min(minor, std::max<int64_t>(1, limit / 2 / per_res) * kOzBlock);
+  p->panels = (minor + w - 1) / w;
+  p->w = round_up((minor + p->panels - 1) / p->panels, kOzBlock);
+  const int64_t res_bytes = per_res * (p->w / kOzBlock);
+  p->per_mod = (major + p->w) * plan.Kp * 2;
+  p->G = std::min<int64_t>(kCrtModuli, (limit - res_bytes) / p->per_mod);
+  if (p->G < 1) return false;
+  p->need[0] = oz_scale_bytes(plan.Mp, plan.Np, plan.K);
+  p->need[1] = (size_t)(p->G * p->per_mod);
+  p->need[2] = (size_t)res_bytes;
+  return true;
+}
+
+// Takes the scratch.  What is not there yet is taken only outside a stream
+// capture, and only where it leaves as much memory free as it takes.
+bool exact_scratch(uvatrmm_handle_t h, const ExactPlan &p) {
   size_t grow = 0;
   for (int k = 0; k < 3; ++k)
-    if (h->ws_cap[4 + k] < need[k]) grow += need[k];
+    if (h->ws_cap[4 + k] < p.need[k]) grow += p.need[k];
   if (grow) {
-    if (stream_captures(h)) return UVATRMM_OK;
+    if (stream_captures(h)) return false;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b / 2 < grow) {
       cudaGetLastError();
-      return UVATRMM_OK;
+      return false;
     }
   }
-  void *e = workspace(h, 4, need[0]);
-  uint16_t *planes = e ? static_cast<uint16_t *>(workspace(h, 5, need[1])) : nullptr;
-  uint16_t *res = planes ? static_cast<uint16_t *>(workspace(h, 6, need[2])) : nullptr;
-  if (!res) return ok();
+  for (int k = 0; k < 3; ++k)
+    if (!workspace(h, 4 + k, p.need[k])) {
+      ok();
+      return false;
+    }
+  return true;
+}
+
+}  // namespace
+
+void exact_reserve(uvatrmm_handle_t h, int64_t M, int64_t N, int64_t K, bool by_cols) {
+  ExactPlan p;
+  if (exact_plan(h, M, N, K, by_cols, &p)) exact_scratch(h, p);
+}
+
+int exact_product(uvatrmm_handle_t h, const OzOperand &L, const OzOperand &R, bool tri_none, bool tri_left,
+                  bool tri_lower, double alpha, double beta, double *C, int64_t ldc, const OzCtl **gate, double *stage,
+                  int64_t lds) {
+  *gate = nullptr;
+  const bool by_cols = tri_left;  // the minor dimension: columns of Rgt, else rows of Lft
+  ExactPlan p;
+  if (!exact_plan(h, L.P, R.P, L.K, by_cols, &p) || !exact_scratch(h, p)) return UVATRMM_OK;
+  const OzPlan &plan = p.plan;
+  const int64_t w = p.w, G = p.G;
+  void *e = h->ws[4];
+  uint16_t *planes = static_cast<uint16_t *>(h->ws[5]), *res = static_cast<uint16_t *>(h->ws[6]);
   OzCtl *ctl = handle_ctl(h);
   const OzScaleBuf sb = oz_scale_buf(e, plan.Mp, plan.Np, plan.K);
   bool sliced = false;
   int rc = UVATRMM_OK;
-  if (panels == 1 && G == plan.n_moduli)
+  if (p.panels == 1 && G == plan.n_moduli)
     rc = oz_prep_once(L, R, sb, plan, ctl, h->dctl, fused_slots(h), planes, planes + G * plan.Mp * plan.Kp,
                       h->dctl + 1, h->num_sms, h->exchange_expiry_polls, h->stream, &sliced);
   if (rc == UVATRMM_OK && !sliced) rc = oz_scales(L, R, sb, scale_counters(h), ctl, h->dctl, h->stream);
