@@ -163,3 +163,101 @@ def test_a_products_time_holds_no_allocation(built, n):
         h.close()
     warm.close()
     assert np.median(first) <= 2 * np.median(later), (first, later)
+
+
+def triangle(A, uplo, trans):
+    """op(A) as a host matrix from the column-major device tensor."""
+    x = A.cpu().numpy().T
+    x = np.tril(x) if uplo == LOWER else np.triu(x)
+    return x.T if trans == TRANS else x
+
+
+def assert_within_fp64(got, side, T, B, alpha, want, where):
+    """Entry by entry within 8 k eps of |alpha| |op(A)| |B| of the double-double oracle."""
+    k = T.shape[0]
+    room = 8 * k * EPS * abs(alpha) * (np.abs(T) @ np.abs(B) if side == LEFT else np.abs(B) @ np.abs(T))
+    assert np.all(np.abs(got - want)[where] <= room[where])
+
+
+# (By the repository's rule the small kernel stands behind the route at these
+# sizes, split along K at the first three.)
+@pytest.mark.parametrize("ka,vecs", [(300, 300), (217, 401), (2500, 12), (700, 300)])
+@pytest.mark.parametrize("side,uplo,trans", [(LEFT, LOWER, NOTRANS), (LEFT, UPPER, TRANS), (RIGHT, UPPER, NOTRANS),
+                                             (RIGHT, LOWER, TRANS), (LEFT, UPPER, NOTRANS)])
+@pytest.mark.parametrize("what", ["span", "nan"])
+def test_declined_calls_are_right(built, ka, vecs, side, uplo, trans, what):
+    """Operands that the route cannot hold, at sizes where a split kernel
+    computes the call: in place, out of place and on host memory."""
+    h = u.Handle()
+    m, n = (ka, vecs) if side == LEFT else (vecs, ka)
+    try:
+        A, lda, B, ldb = operands(side, uplo, m, n, "uniform", pad=1)
+        row, col = m // 3, n // 2
+        B[col, row] = 2.0 ** 300 if what == "span" else float("nan")
+        T = triangle(A, uplo, trans)
+        hB = B.cpu().numpy()[:, :m].T.copy()
+        where = np.ones((m, n), bool)
+        if what == "nan":  # the line that holds it
+            where[(slice(None), col) if side == LEFT else (row, slice(None))] = False
+        # (The oracle multiplies by the zeros of the triangle: a zero in place of the NaN.)
+        want = oracle_dd(side, uplo, trans, m, n, -0.75, A, lda, B.nan_to_num(0.0), ldb)
+        got = [run(h, side, uplo, trans, NONUNIT, m, n, -0.75, A, lda, B, ldb, in_place) for in_place in (True, False)]
+        host = B.cpu().numpy().ravel().copy()
+        h.dtrmm(COL, side, uplo, trans, NONUNIT, m, n, -0.75, A.cpu().numpy().ravel(), lda, host, ldb)
+        got.append(host.reshape(n, ldb))
+        hB[np.isnan(hB)] = 0.0
+        for x in got:
+            assert np.all(x[:, m:] == -7.0), "padding was written"
+            C = x[:, :m].T
+            assert_within_fp64(C, side, T, hB, -0.75, want, where)
+            if what == "nan":
+                # Its line: not a number where the entry takes part, right away from there.
+                line = C[:, col] if side == LEFT else C[row, :]
+                true, at = (want[:, col], row) if side == LEFT else (want[row, :], col)
+                takes = T[:, at] != 0.0 if side == LEFT else T[at, :] != 0.0
+                assert not np.isfinite(line[takes]).any()
+                far = ~takes & (np.abs(np.arange(ka) - at) >= 64)
+                assert np.allclose(line[far], true[far], rtol=0, atol=8 * ka * EPS * ka)
+    finally:
+        h.close()
+
+
+@pytest.mark.parametrize("entry", [float("nan"), float("inf"), 2.0 ** 300])
+@pytest.mark.parametrize("layout,ta,tb", [(COL, NOTRANS, NOTRANS), (COL, TRANS, NOTRANS), (101, NOTRANS, TRANS)])
+def test_declined_gemms_and_host_calls_equal_the_pinned_handles(built, layout, ta, tb, entry):
+    """A GEMM whose operands the route cannot hold, odd leading dimensions and
+    beta, and a host TRMM (1100 x 901): the tile kernel's finite results, bit
+    by bit."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    h, pinned = u.Handle(), u.Handle(engine=u.ENGINE_DFMA)
+    m, n, k = 700, 651, 903
+
+    def store(rows, cols):  # (lines of the layout, one entry longer: odd where the length is even)
+        lines, length = (cols, rows) if layout == COL else (rows, cols)
+        ld = length + 1 + length % 2
+        return torch.rand(lines, ld, dtype=torch.float64, device="cuda", generator=gen) * 2 - 1, ld
+
+    A, lda = store(k, m) if ta == TRANS else store(m, k)
+    B, ldb = store(n, k) if tb == TRANS else store(k, n)
+    C, ldc = store(m, n)
+    B[40, 30] = entry
+    try:
+        out = []
+        for hh in (h, pinned):
+            X = C.clone()
+            torch.cuda.synchronize()
+            hh.dgemm_device(layout, ta, tb, m, n, k, -0.5, A, lda, B, ldb, 2.0, X, ldc)
+            hh.sync()
+            host = np.random.default_rng(1).uniform(-1, 1, 1100 * 901)
+            T = np.random.default_rng(2).uniform(-1, 1, 1100 * 1100)
+            host[5000] = entry
+            hh.dtrmm(COL, LEFT, LOWER, ta, NONUNIT, 1100, 901, 1.25, T, 1100, host, 1100)
+            out.append((X.cpu().numpy(), host))
+        for x, y in zip(*out):
+            fine = np.isfinite(y)  # (the tile kernel also multiplies by zeros beside the diagonal)
+            assert np.array_equal(x[fine], y[fine])
+            assert fine.mean() > 0.9
+    finally:
+        h.close()
+        pinned.close()

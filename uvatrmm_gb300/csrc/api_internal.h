@@ -193,7 +193,7 @@ inline int *scale_counters(uvatrmm_handle_t h) {
 enum class Route { kTile, kSmall, kExact };
 Route pick_route(int64_t M, int64_t N, int64_t K, bool tri, bool tri_left, bool in_place = false);
 // Behind the lossless route of a TRMM: the small kernel instead of the tile
-// kernel (the same bits) where it is faster.
+// kernel where it is faster (the same bits where it is not split along K).
 bool small_behind_exact(int64_t M, int64_t N, int64_t K, bool tri_left);
 // True when no option pins the handle's FP64 calls to the tile kernel, nor
 // the schedule and shape of this call.

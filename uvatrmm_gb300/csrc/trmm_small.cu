@@ -14,7 +14,9 @@
 // take 0.07 us per k, so where there are too few outputs for the chip K is
 // split into chunks of kc, each block sums one chunk, and a second launch adds
 // an output's partial sums in the chunks' order.  kc depends on the problem's
-// sizes alone: a call, a group and the server give the same bits.
+// sizes alone: a call, a group and the server give the same bits, unless the
+// partial sums' workspace is not to be had (a first call that is captured, or
+// no memory): then the product runs unsplit, or on the tile kernel.
 //
 // In place unsplit, the blocks of one vector group (all rows, up to 8 x 32) form a
 // cluster: they read the vectors, meet at the cluster's barrier, and only
