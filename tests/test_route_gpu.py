@@ -261,3 +261,42 @@ def test_declined_gemms_and_host_calls_equal_the_pinned_handles(built, layout, t
     finally:
         h.close()
         pinned.close()
+
+
+@pytest.mark.parametrize("on_device", [True, False])
+def test_a_server_reserves_the_moduli_that_fit_and_gives_back_the_rest(built, on_device):
+    """Under 2 GiB a 1500 x 1500 request has planes for 16 moduli: uniform
+    entries (14) take the route, as single calls do; entries of wide spans (some
+    24) and a request too large for any planes run as tiles.  More are sent at
+    once than 2 GiB hold planes for."""
+    import torch
+    h = u.Handle()
+    srv = u.Server(h, hbm_budget_bytes=2 << 30)
+    try:
+        probs = []
+        for i, (n, data) in enumerate([(1500, "uniform")] * 9 + [(1500, "wide"), (5200, "uniform"), (1500, "uniform")]):
+            side = [LEFT, RIGHT][i % 2]
+            A, lda, B, ldb = operands(side, LOWER, n, n, data)
+            probs.append(dict(layout=COL, side=side, uplo=LOWER, transa=NOTRANS, diag=NONUNIT, m=n, n=n, alpha=1.0, A=A,
+                              lda=lda, B=B.clone(), B0=B, ldb=ldb, tier=u.TIER_FP64, moduli=0, data=data))
+        want = [run(h, p["side"], LOWER, NOTRANS, NONUNIT, p["m"], p["m"], 1.0, p["A"], p["lda"], p["B0"], p["ldb"],
+                    in_place=False) for p in probs]
+        torch.cuda.synchronize()
+        for _ in range(2):
+            for p in probs:
+                p["B"].copy_(p["B0"])
+            torch.cuda.synchronize()
+            sent = probs if on_device else [dict(p, A=p["A"].cpu().numpy(), B=p["B0"].cpu().numpy()) for p in probs]
+            for rid in [srv.submit(p, on_device=on_device) for p in sent]:
+                assert srv.wait(rid) == 0
+            for p, q, w in zip(probs, sent, want):
+                got = q["B"].cpu().numpy() if on_device else q["B"]
+                if p["m"] == 1500 and p["data"] == "uniform":
+                    assert np.array_equal(got, w)
+                else:
+                    assert not np.array_equal(got, w)
+                    assert np.linalg.norm(got - w) <= 8 * p["m"] * EPS * np.linalg.norm(w)
+        assert srv.stats()["peak_bytes"] <= 2 << 30
+    finally:
+        srv.close()
+        h.close()

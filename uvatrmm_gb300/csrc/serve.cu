@@ -7,7 +7,8 @@
 //            stream; FP64 requests large enough for the lossless integer
 //            route have their operands scaled there, and once the decision
 //            is back on the host they are Ozaki work (with the moduli they
-//            need) or, where it says no, FP64 tiles;
+//            need: the rest of their planes goes back to the pool) or, where
+//            it says no, FP64 tiles;
 //   tick   - one grouped launch per kind over tile ranges taken from every
 //            active request (Ozaki slicing of newly admitted requests, the
 //            residue GEMM, Ozaki reassembly of requests whose last GEMM tiles
@@ -43,6 +44,8 @@ double now_s() {
   return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
 
+size_t pool_round(size_t bytes) { return (bytes + 255) / 256 * 256; }
+
 // First-fit allocator over [0, size) with 256-byte granularity.
 class Pool {
  public:
@@ -53,7 +56,7 @@ class Pool {
     used_ = peak_ = 0;
   }
   bool alloc(size_t bytes, size_t *off) {
-    bytes = (bytes + 255) / 256 * 256;
+    bytes = pool_round(bytes);
     for (auto it = free_.begin(); it != free_.end(); ++it) {
       if (it->second >= bytes) {
         *off = it->first;
@@ -68,7 +71,7 @@ class Pool {
     return false;
   }
   void release(size_t off, size_t bytes) {
-    bytes = (bytes + 255) / 256 * 256;
+    bytes = pool_round(bytes);
     used_ -= bytes;
     auto it = free_.emplace(off, bytes).first;
     auto nx = std::next(it);
@@ -120,6 +123,7 @@ struct Req {
   bool exact = false, deciding = false;
   int ctl_slot = -1;
   OzCtl *ctl = nullptr;
+  size_t planes_at = 0;  // its planes' place in the pool block; given back from there on as the decision allows
   double *stage_b = nullptr;  // where B's copy goes if it becomes FP64 tiles
   int lane = 0;               // its copy stream
   cudaStream_t copy = nullptr;
@@ -222,7 +226,7 @@ size_t working_bytes(const Req &r) {
   const Trmm &t = r.t;
   const int64_t ka = t.side == CblasLeft ? t.m : t.n;
   size_t b = 0;
-  auto add = [&](size_t x) { b += (x + 255) / 256 * 256; };
+  auto add = [&](size_t x) { b += pool_round(x); };
   const bool tier_oz = r.p.tier == UVATRMM_TIER_OZAKI;
   if (stages_a(r)) add((size_t)round_up(ka, 16) * ka * 8);
   if (!tier_oz) {
@@ -287,10 +291,13 @@ int setup_tiles(Req &r) {
   return UVATRMM_OK;
 }
 
-// The residue GEMM's descriptor, for plan.n_moduli moduli.
-int setup_residues(uvatrmm_server_t s, Req &r) {
+// Lays the planes and product residues of plan.n_moduli moduli out from
+// `planes` on and builds the residue GEMM's descriptor.
+int setup_residues(uvatrmm_server_t s, Req &r, char *planes) {
   const Trmm &t = r.t;
   const OzPlan &pl = r.plan;
+  r.LR = reinterpret_cast<uint16_t *>(planes);
+  r.res = reinterpret_cast<uint16_t *>(planes + pool_round(oz_bytes(pl, pl.n_moduli, r.exact).planes));
   OzGemmLaunch L;
   L.LR = r.LR;
   L.RR = r.RR = r.LR + (int64_t)pl.n_moduli * pl.Mp * pl.Kp;
@@ -320,7 +327,7 @@ int setup(uvatrmm_server_t s, Req &r) {
   size_t cur = 0;
   auto take = [&](size_t x) {
     char *p = base + cur;
-    cur += (x + 255) / 256 * 256;
+    cur += pool_round(x);
     return p;
   };
   const bool tier_oz = r.p.tier == UVATRMM_TIER_OZAKI;
@@ -367,8 +374,9 @@ int setup(uvatrmm_server_t s, Req &r) {
     const OzBytes o = oz_bytes(pl, pl.n_moduli, r.exact);
     r.sb = oz_scale_buf(take(o.scale), pl.Mp, pl.Np, pl.K);
     r.ctl = r.exact ? reinterpret_cast<OzCtl *>(take(o.ctl)) : nullptr;
-    r.LR = reinterpret_cast<uint16_t *>(take(o.planes));
-    r.res = reinterpret_cast<uint16_t *>(take(o.res));
+    r.planes_at = cur;
+    take(o.planes);
+    take(o.res);
   }
   if (r.exact) {
     // Scaled and decided behind the copies; the host reads the decision.
@@ -383,7 +391,7 @@ int setup(uvatrmm_server_t s, Req &r) {
             cudaSuccess)
       return UVATRMM_EDEVICE;
     r.h2d_pending = r.deciding = true;
-  } else if (int rc = tier_oz ? setup_residues(s, r) : setup_tiles(r)) {
+  } else if (int rc = tier_oz ? setup_residues(s, r, base + r.planes_at) : setup_tiles(r)) {
     return rc;
   }
   if (r.h2d_pending) {
@@ -399,10 +407,19 @@ int decided(uvatrmm_server_t s, Req &r) {
   const OzCtl c = s->ctl_host[r.ctl_slot];
   s->ctl_free.push_back(r.ctl_slot);
   r.ctl_slot = -1;
-  if (c.go) {
+  const bool go = c.go && c.n <= r.plan.n_moduli;
+  size_t keep = r.planes_at;
+  if (go) {
     r.plan.n_moduli = c.n;
-    return setup_residues(s, r);
+    const OzBytes o = oz_bytes(r.plan, c.n, true);
+    keep += pool_round(o.planes) + pool_round(o.res);
   }
+  {
+    std::lock_guard<std::mutex> lk(s->mu);
+    if (keep < r.bytes) s->pool.release(r.off + keep, r.bytes - keep);
+    r.bytes = keep;
+  }
+  if (go) return setup_residues(s, r, s->arena + r.off + r.planes_at);
   r.small = small_behind_exact(r.t.m, r.t.n, r.plan.K, r.t.side == CblasLeft);
   if (r.Bin != r.stage_b) {
     const int64_t lb = round_up(r.t.m, 16);
@@ -421,6 +438,8 @@ void finish(uvatrmm_server_t s, Req &r, int status) {
   r.state = status == UVATRMM_OK ? DONE : FAILED;
   r.status = status;
   r.t_done = now_s();
+  // (What was enqueued for a request that fails may still use its memory.)
+  if (status != UVATRMM_OK && r.copy) cudaStreamSynchronize(r.copy);
   if (r.bytes) s->pool.release(r.off, r.bytes);
   r.bytes = 0;
   if (r.ctl_slot >= 0) s->ctl_free.push_back(r.ctl_slot);
@@ -439,7 +458,7 @@ void finish(uvatrmm_server_t s, Req &r, int status) {
 }
 
 // Bytes an area of a tick slot takes (descriptors start at multiples of 256).
-size_t slot_area(size_t bytes) { return (bytes + 255) / 256 * 256; }
+size_t slot_area(size_t bytes) { return pool_round(bytes); }
 
 // Builds and enqueues one tick; returns false when there was nothing to do.
 bool launch_tick(uvatrmm_server_t s, std::vector<Req *> &act) {
@@ -870,10 +889,12 @@ UVATRMM_API int uvatrmm_server_submit(uvatrmm_server_t s, const uvatrmm_trmm_pro
     return ok();
   }
   // The lossless route takes at most an eighth of the budget per request, so
-  // that it does not narrow how many are admitted at once by much.
+  // that it does not narrow how many are admitted at once by much: planes for
+  // as many moduli as that holds (which depends on the request alone, so that
+  // its result does, too), until the decision tells how many are needed.
   r->bytes = working_bytes(*r);
-  if (r->exact && (int64_t)r->bytes > s->cfg.hbm_budget_bytes / 8) {
-    r->exact = false;
+  while (r->exact && (int64_t)r->bytes > s->cfg.hbm_budget_bytes / 8) {
+    r->exact = --pl.n_moduli >= 2;
     r->bytes = working_bytes(*r);
   }
   std::lock_guard<std::mutex> lk(s->mu);
