@@ -142,7 +142,9 @@ UVATRMM_API int uvatrmm_set_option(uvatrmm_handle_t handle, int option, int valu
 
 /* ---------------------------------------------------------------- TRMM */
 /* Host buffers, in place on B, with status.  handle may be NULL (a
- * per-thread default handle on the current device is used). */
+ * per-thread default handle on the current device is used; when a thread
+ * other than the process's first ends, its default handle goes, unless groups
+ * or captured calls use it). */
 UVATRMM_API int uvatrmm_dtrmm(uvatrmm_handle_t handle, int layout, int side, int uplo, int transa, int diag,
                               int64_t m, int64_t n, double alpha, const double *A, int64_t lda, double *B,
                               int64_t ldb);

@@ -1,5 +1,8 @@
 // C ABI of libuvatrmm.so: handles, argument checking, CBLAS row-major
 // normalisation, operand staging, and the plain FP64 TRMM entry points.
+#include <sys/syscall.h>
+#include <unistd.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -14,9 +17,22 @@
 
 namespace uvt {
 
+static void retire_default(uvatrmm_handle_t h);
+
 static thread_local int tl_status = UVATRMM_OK;
 static thread_local std::string tl_msg;
-static thread_local uvatrmm_handle_t tl_default[64] = {};
+
+// A thread's default handles, one per device.  A thread that ends gives their
+// memory back; the process's first thread ends with the process, which does.
+struct DefaultHandles {
+  uvatrmm_handle_t h[64] = {};
+  ~DefaultHandles() {
+    if ((pid_t)syscall(SYS_gettid) == getpid()) return;
+    for (auto &d : h)
+      if (d) retire_default(d);
+  }
+};
+static thread_local DefaultHandles tl_default;
 
 int fail(int status, const std::string &msg) {
   tl_status = status;
@@ -45,12 +61,14 @@ uvatrmm_handle_t resolve(uvatrmm_handle_t h) {
     fail(UVATRMM_EDEVICE, "no CUDA device");
     return nullptr;
   }
-  if (!tl_default[dev]) {
+  if (!tl_default.h[dev]) {
     uvatrmm_handle_t nh = nullptr;
     if (uvatrmm_create(&nh) != UVATRMM_OK) return nullptr;
-    tl_default[dev] = nh;
+    tl_default.h[dev] = nh;
   }
-  return tl_default[dev];
+  h = tl_default.h[dev];
+  h->captured |= stream_captures(h);
+  return h;
 }
 
 namespace {
@@ -116,6 +134,42 @@ bool small_scratch(uvatrmm_handle_t h, SmallProduct *p) {
   ok();
   p->kc = 0;
   return p->K <= kSmallMaxK;
+}
+
+// (Its work is done, or cudaFree waits for it.)
+static void free_handle(uvatrmm_handle_t h) {
+  for (int i = 0; i < uvatrmm_handle_st::kSlots; ++i)
+    if (h->ws[i]) cudaFree(h->ws[i]);
+  for (void *p : h->ws_kept) cudaFree(p);
+  if (h->dctl) cudaFree(h->dctl);
+  if (h->ev0) cudaEventDestroy(h->ev0);
+  if (h->ev1) cudaEventDestroy(h->ev1);
+  release_host_staging(h);
+  for (auto &ev : h->sev)
+    if (ev) cudaEventDestroy(ev);
+  delete h;
+}
+
+// (Not by its stream, which may be gone by now.)
+static void retire_default(uvatrmm_handle_t h) {
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess || (dev != h->device && cudaSetDevice(h->device) != cudaSuccess)) {
+    cudaGetLastError();
+    return;
+  }
+  CaptureModeRelaxed relaxed;
+  if (!h->captured && h->groups == 0) {
+    free_handle(h);
+    return;
+  }
+  // Graphs use the handle: what they do not use goes.
+  for (int i = 0; i < uvatrmm_handle_st::kSlots; ++i)
+    if (h->ws[i] && !h->ws_captured[i]) {
+      cudaFree(h->ws[i]);
+      h->ws[i] = nullptr;
+      h->ws_cap[i] = 0;
+    }
+  release_host_staging(h);
 }
 
 int collect_status(uvatrmm_handle_t h) {
@@ -445,18 +499,9 @@ UVATRMM_API int uvatrmm_create(uvatrmm_handle_t *handle) {
 UVATRMM_API int uvatrmm_destroy(uvatrmm_handle_t h) {
   if (!h) return ok();
   cudaStreamSynchronize(h->stream);
-  for (int i = 0; i < uvatrmm_handle_st::kSlots; ++i)
-    if (h->ws[i]) cudaFree(h->ws[i]);
-  for (void *p : h->ws_kept) cudaFree(p);
-  if (h->dctl) cudaFree(h->dctl);
-  if (h->ev0) cudaEventDestroy(h->ev0);
-  if (h->ev1) cudaEventDestroy(h->ev1);
-  release_host_staging(h);
-  for (auto &ev : h->sev)
-    if (ev) cudaEventDestroy(ev);
-  for (auto &d : tl_default)
+  for (auto &d : tl_default.h)
     if (d == h) d = nullptr;
-  delete h;
+  free_handle(h);
   return ok();
 }
 

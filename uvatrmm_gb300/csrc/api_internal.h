@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -43,6 +44,10 @@ struct uvatrmm_handle_st {
   // that were outgrown: kept until the handle goes, as a graph may use them.
   bool ws_captured[kSlots] = {};
   std::vector<void *> ws_kept;
+  // What keeps a default handle when its thread ends: groups alive on it, or
+  // calls on it that were captured.
+  std::atomic<int> groups{0};
+  bool captured = false;
   // [0] tile counter, [1] kernel status word, [2], [3] the server's tile
   // counters; the lossless route's OzCtl at kHandleCtlOffset, the scaling's
   // counters at kHandleCountersOffset, its blocks' words at kHandleSlotsOffset.

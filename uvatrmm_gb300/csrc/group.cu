@@ -565,6 +565,7 @@ UVATRMM_API int uvatrmm_group_create(uvatrmm_handle_t h, const uvatrmm_trmm_prob
     return rc;
   }
   *group = g;
+  h->groups++;
   return ok();
 }
 
@@ -592,6 +593,7 @@ UVATRMM_API int uvatrmm_group_destroy(uvatrmm_group_t g) {
   {
     std::lock_guard<std::mutex> lk(g->h->mu);
     cudaStreamSynchronize(g->h->stream);
+    g->h->groups--;
   }
   destroy_group(g);
   return ok();
