@@ -300,3 +300,31 @@ def test_a_server_reserves_the_moduli_that_fit_and_gives_back_the_rest(built, on
     finally:
         srv.close()
         h.close()
+
+
+@pytest.mark.parametrize("side,ka,vecs", [(LEFT, 5000, 60), (RIGHT, 3293, 135)])
+def test_declined_calls_take_little_longer_than_the_tile_kernel(built, side, ka, vecs):
+    """At most 30 % (the scaling and the launches that return at once are 30 us
+    of 275 at the smallest; kernels that found the chip unevenly occupied, or
+    the slower of the two, took 40 to 70 % more)."""
+    import torch
+    m, n = (ka, vecs) if side == LEFT else (vecs, ka)
+    A, lda, B, ldb = operands(side, LOWER, m, n, "uniform")
+    B[n // 2, m // 2] = float("nan")
+    out = torch.zeros_like(B)
+    took = []
+    for options in ({}, {"engine": u.ENGINE_DFMA}):
+        h = u.Handle(**options)
+        times = []
+        for _ in range(7):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            e0.record()
+            for _ in range(5):
+                h.dtrmm_device_oop(COL, side, LOWER, NOTRANS, NONUNIT, m, n, 1.0, A, lda, B, ldb, out, ldb)
+            e1.record()
+            torch.cuda.synchronize()
+            times.append(e0.elapsed_time(e1))
+        h.close()
+        took.append(np.median(times[2:]))
+    assert took[0] <= 1.3 * took[1], took
