@@ -391,6 +391,7 @@ int device_trmm(uvatrmm_handle_t h, int layout, int side, int uplo, int transa, 
   if (gate && small_behind_exact(t.m, t.n, ka, t.side == CblasLeft)) {
     sp = small_trmm(t, A, la, B, lb, dC, ldc, beta);
     sp.gate = gate;
+    sp.counter = h->dctl;
   }
   if (sp.gate && small_scratch(h, &sp)) rc = launch_small(sp, false, h->stream);
   else rc = run_fp64(h, t, A, la, B, lb, dC, ldc, schedule, shape, beta, gate);
@@ -438,6 +439,7 @@ int host_trmm(uvatrmm_handle_t h, int layout, int side, int uplo, int transa, in
   if (small) {
     sp = small_trmm(t, dA, la, dB, lb, dC, lb, 0.0);
     sp.gate = gate;
+    sp.counter = h->dctl;
   }
   if (small && small_scratch(h, &sp)) {
     if ((rc = launch_small(sp, false, h->stream)) != UVATRMM_OK)

@@ -151,6 +151,7 @@ struct SmallProduct {
   int kc;        // split: k per chunk (small_chunk()), 0 unsplit
   double *part;  // split: partial sums, small_part_bytes()
   const struct OzCtl *gate;  // lossless route in front: nothing to do where it computed the result
+  int *counter;              // with `gate` in a launch of its own: zeroed by the route's scaling
 };
 constexpr int kSmallMaxK = 2048;  // of an unsplit product (its vectors lie in shared memory)
 int small_chunk(int64_t R, int64_t V, int64_t K, bool tri);

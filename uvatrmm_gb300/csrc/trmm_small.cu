@@ -144,20 +144,27 @@ __global__ void __launch_bounds__(kThreads) trmm_small_kernel(const __grid_const
                       (int)blockIdx.z, vs);
 }
 
-// Behind the lossless route: mostly there is nothing to do, so few blocks,
-// which otherwise take several units each (m = n = 1000: 9.9 us for 8000
-// blocks that return at once).
+// Behind the lossless route: mostly there is nothing to do, so few blocks
+// (m = n = 1000: 9.9 us for 8000 that return at once).  They take their units
+// from the call's counter: dealt out in turns, those of the blocks that are not
+// resident at first (1216 of seven per SM, fewer by shared memory from K = 500
+// on) ran last on a chip otherwise idle (768 x 2564: 1626 -> 1367 us, 65 x 30730 402 -> 325).
 constexpr int kGatedBlocks = 1216;
 __global__ void __launch_bounds__(kThreads) trmm_small_gated_kernel(const __grid_constant__ SmallProduct p) {
   extern __shared__ double vs[];
+  __shared__ int next;
   chain_wait();
   if (p.gate->go) return;
   const int nx = (p.R + kRows - 1) / kRows, ny = (p.V + kVecs - 1) / kVecs;
   const int units = nx * ny * (p.kc ? (p.K + p.kc - 1) / p.kc : 1);
-  for (int i = (int)blockIdx.x; i < units; i += (int)gridDim.x) {
-    if (i != (int)blockIdx.x) __syncthreads();  // the unit before has read its vectors
+  for (;;) {
+    if (threadIdx.x == 0) next = atomicAdd(p.counter, 1);
+    __syncthreads();
+    const int i = next;
+    if (i >= units) return;
     const int y = i / nx % ny, z = i / nx / ny;
     small_body<false>(p, rotated(i % nx, y + z, nx), y, z, vs);
+    __syncthreads();  // the unit has read its vectors
   }
 }
 
