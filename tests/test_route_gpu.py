@@ -302,7 +302,8 @@ def test_a_server_reserves_the_moduli_that_fit_and_gives_back_the_rest(built, on
         h.close()
 
 
-@pytest.mark.parametrize("side,ka,vecs", [(LEFT, 5000, 60), (RIGHT, 3293, 135), (LEFT, 65, 30730), (RIGHT, 768, 2564)])
+@pytest.mark.parametrize("side,ka,vecs", [(LEFT, 5000, 60), (RIGHT, 3293, 135), (LEFT, 65, 30730), (RIGHT, 768, 2564),
+                                          (LEFT, 120, 14785)])
 def test_declined_calls_take_little_longer_than_the_tile_kernel(built, side, ka, vecs):
     """At most 30 % (the scaling and the launches that return at once are 30 us
     of 275 at the smallest; kernels that found the chip unevenly occupied, or
