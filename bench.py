@@ -52,8 +52,10 @@ FP64_FLOP_PER_CLK_SM = 4.0
 # dram__bytes_write.sum, first launch, cold L2) with the banded tile order:
 # 1.73x, 4.23x and 8.67x the algorithmic bytes 8 (m(m+1)/2 + 2 m n).
 TRAFFIC_MEASURED = {4096: 0.5810e9, 8192: 5.6793e9, 16384: 46.5478e9}
-# The same of all launches of one call with default options (lossless route), warm.
-ROUTE_TRAFFIC = {4096: 2.9564e9}
+# The same of all launches of one call with default options (lossless route; 4096 warm, 16384 cold).
+ROUTE_TRAFFIC = {4096: 2.9550e9, 16384: 223.7e9}
+ROUTE_TRAFFIC_SOURCE = ("ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum python -m uvatrmm_gb300.run_case "
+                        "--tier fp64 --engine default --m M --reps 1 (one pass), all launches of a call")
 TRAFFIC_SOURCE = ("ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum -k regex:trmm_fp64_kernel -c 1 "
                   "python -m uvatrmm_gb300.run_case --tier fp64 --m M --reps 1 (one pass), per launch")
 
@@ -374,6 +376,7 @@ def run_gpu(args, ws, rank, local):
         "roofline": {"bound": "tensor", "achieved": round(mma_tflops, 2), "peak": bf16, "unit": "TFLOP/s",
                      "frac": round(mma_tflops / bf16, 4), "peak_source": bf16_src, "traffic": ROUTE_TRAFFIC.get(m) if m == n else None,
                      "traffic_measured": {f"m=n={k}": v for k, v in ROUTE_TRAFFIC.items()},
+                     "traffic_source": ROUTE_TRAFFIC_SOURCE,
                      "flops": f"bf16 MMA flops of {moduli} residue products (tile-exact) / mean time of the whole "
                               "call (scaling, slicing, products, reassembly)"},
         "plain_fp64": plain,
@@ -403,9 +406,12 @@ def count_launches(call, h):
 
 def exact_moduli(k, b0, b1):
     """Moduli that the lossless route takes for integers of b0 and b1 bits: the fewest with K 2^(b0 + b1) <= 0.47 M
-    (the seeded uniform entries are multiples of 2^-52 below 1)."""
+    (the seeded uniform entries are multiples of 2^-52 below 1).  The device decides; this is its rule over the
+    kernels' own list of moduli, for the operation count."""
     import math
-    mods = [363, 362, 361, 359, 355, 353, 349, 347, 343, 337, 331, 317, 313, 311, 307, 299, 293, 289]
+    import re
+    with open(os.path.join(ROOT, "uvatrmm_gb300", "csrc", "ozaki.cuh")) as f:
+        mods = [int(x) for x in re.search(r"kModuli\[kCrtModuli\] = \{([^}]*)\}", f.read()).group(1).split(",")]
     need, have = math.log2(k) + b0 + b1 - math.log2(0.47), 0.0
     for n, m in enumerate(mods, 1):
         have += math.log2(m)

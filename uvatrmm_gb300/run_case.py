@@ -1,13 +1,17 @@
 """Runs one TRMM configuration a few times through the C ABI (for profilers).
 
     python -m uvatrmm_gb300.run_case --tier fp64 --engine dmma --m 4096 --n 4096 --reps 2
+    python -m uvatrmm_gb300.run_case --tier fp64 --engine default --m 4096 --reps 2
     python -m uvatrmm_gb300.run_case --tier ozaki --m 6144 --reps 2
 
 Operands are seeded uniform[-1,1) (column-major, device-resident, generated
 by the library); the product is B := op(A) B (side Left) or B op(A) (side
 Right), out of place for the FP64 tier and in place for the Ozaki tier.
-Prints the mean wall time per call after one untimed call; the kernels'
-own time is what a profiler reads.
+The engine `default` leaves the handle's options alone, so that an FP64 call
+takes its own route (the lossless integer products, the small kernel or the
+tile kernel); `dfma` and `dmma` pin it to the tile kernel.  Prints the mean
+wall time per call after one untimed call; the kernels' own time is what a
+profiler reads.
 """
 from __future__ import annotations
 
@@ -18,7 +22,7 @@ import time
 def main() -> None:
     ap = argparse.ArgumentParser()
     ap.add_argument("--tier", choices=["fp64", "ozaki"], default="fp64")
-    ap.add_argument("--engine", choices=["dfma", "dmma"], default="dfma")
+    ap.add_argument("--engine", choices=["dfma", "dmma", "default"], default="dfma")
     ap.add_argument("--m", type=int, default=4096)
     ap.add_argument("--n", type=int, default=0, help="0: same as m")
     ap.add_argument("--side", choices=["L", "R"], default="L")
@@ -37,7 +41,8 @@ def main() -> None:
     trans = u.NOTRANS if a.trans == "N" else u.TRANS
     ka = m if side == u.LEFT else n
     h = u.Handle()
-    h.set_option("engine", u.ENGINE_DMMA if a.engine == "dmma" else u.ENGINE_DFMA)
+    if a.engine != "default":
+        h.set_option("engine", u.ENGINE_DMMA if a.engine == "dmma" else u.ENGINE_DFMA)
     dA = torch.empty(ka * ka, dtype=torch.float64, device="cuda")
     dB = torch.empty(m * n, dtype=torch.float64, device="cuda")
     h.gen_uniform(1, 0, ka, ka, dA, 1, ka, tri=a.uplo)
