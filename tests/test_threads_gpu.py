@@ -223,3 +223,27 @@ def test_calls_from_several_threads(built):
 
     in_threads(6, work)
     h.close()
+
+
+def test_small_calls_beside_another_streams_long_kernel(built):
+    """Calls whose scaling is one launch with an exchange between its blocks,
+    while a pinned handle's tile kernel (some 0.2 s) holds the SMs."""
+    import torch
+    n, big = 512, 6000
+    A, B = (torch.rand(n, n, dtype=torch.float64, device="cuda") for _ in range(2))
+    X, Y = (torch.rand(big, big, dtype=torch.float64, device="cuda") for _ in range(2))
+    Z, want = torch.zeros_like(Y), torch.zeros_like(B)
+    one, two = torch.cuda.Stream(), torch.cuda.Stream()
+    h, pinned = u.Handle(stream=one), u.Handle(stream=two, engine=u.ENGINE_DFMA)
+    out = [torch.zeros_like(B) for _ in range(30)]
+    torch.cuda.synchronize()
+    h.dtrmm_device_oop(COL, LEFT, LOWER, NOTRANS, NONUNIT, n, n, 1.0, A, n, B, n, want, n)
+    h.sync()
+    pinned.dtrmm_device_oop(COL, LEFT, LOWER, NOTRANS, NONUNIT, big, big, 1.0, X, big, Y, big, Z, big)
+    for C in out:
+        h.dtrmm_device_oop(COL, LEFT, LOWER, NOTRANS, NONUNIT, n, n, 1.0, A, n, B, n, C, n)
+    h.sync()
+    pinned.sync()
+    assert all(torch.equal(C, want) for C in out)
+    h.close()
+    pinned.close()

@@ -693,7 +693,9 @@ __global__ void __launch_bounds__(256, 3) residue_kernel(const __grid_constant__
 // tier 512 x 512 30.3 -> 23.5, which needs no exchange).
 constexpr int FR = 8;    // rows per block
 constexpr int NT = 512;  // threads; 16 warps have an SM's slicing well in flight
-constexpr uint32_t kFusedSpin = 1u << 21;
+// Polls of the wait for the other blocks, as of every wait here: blocks whose
+// SM another stream's long kernel still holds start that much later.
+constexpr uint32_t kFusedSpin = kSpinLimit;
 constexpr unsigned kLostBlock = 1u << 16;  // OzCtl::done counts blocks below this, blocks whose wait ran out above
 static_assert(kFusedSlots < (int)kLostBlock, "");
 
