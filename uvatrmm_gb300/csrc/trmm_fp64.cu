@@ -512,13 +512,9 @@ __global__ void __launch_bounds__(Cfg<BM>::THREADS, Cfg<BM>::MIN_BLOCKS)
       };
       if (!p.sched_static) {
         const int total = p.n_major * p.n_minor;
-        // A tile per CTA: by its number, as CTAs that start together (behind the
-        // lossless route) would draw two of the longest on one SM.  (1500 x 700:
-        // 3.09 -> 2.20 ms, 1000 x 1000 1.98 -> 1.39; first tiles by number where
-        // there are more than CTAs lose, 2000 x 2000 7.18 -> 7.34.)
-        const bool one = (int)gridDim.x >= total;
-        for (int t = one ? (int)blockIdx.x : atomicAdd(p.counter, 1); ok && t < total;
-             t = one ? total : atomicAdd(p.counter, 1)) {
+        while (ok) {
+          int t = atomicAdd(p.counter, 1);
+          if (t >= total) break;
           int ti, tj;
           decode_dynamic(p, t, ti, tj);
           ok = issue_tile(ti, tj);
@@ -742,18 +738,19 @@ __global__ void __launch_bounds__(Cfg<BM>::THREADS, Cfg<BM>::MIN_BLOCKS)
 }
 
 template <int BM, bool LK, bool RK, template <int> class EngineT>
-int launch_variant(const CUtensorMap &tmL, const CUtensorMap &tmR, const KParams &kp, int grid, bool chained,
+int launch_variant(const CUtensorMap &tmL, const CUtensorMap &tmR, const KParams &kp, int grid, bool alone,
                    cudaStream_t stream) {
   auto kern = trmm_fp64_kernel<BM, LK, RK, EngineT>;
+  constexpr size_t kAlone = std::max<size_t>(Cfg<BM>::SMEM, 116 << 10);  // over half of an SM's 228 KB
   static bool attr_set = false;  // per instantiation
   if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<BM>::SMEM) !=
-        cudaSuccess)
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAlone) != cudaSuccess)
       return UVATRMM_EDEVICE;
     attr_set = true;
   }
-  if (chained)
-    return launch_chained(kern, dim3(grid), dim3(Cfg<BM>::THREADS), Cfg<BM>::SMEM, stream, tmL, tmR, kp) == cudaSuccess
+  if (kp.gate)
+    return launch_chained(kern, dim3(grid), dim3(Cfg<BM>::THREADS), alone ? kAlone : Cfg<BM>::SMEM, stream, tmL, tmR,
+                          kp) == cudaSuccess
                ? UVATRMM_OK
                : UVATRMM_EDEVICE;
   kern<<<grid, Cfg<BM>::THREADS, Cfg<BM>::SMEM, stream>>>(tmL, tmR, kp);
@@ -762,11 +759,11 @@ int launch_variant(const CUtensorMap &tmL, const CUtensorMap &tmR, const KParams
 
 template <int BM, template <int> class EngineT>
 int dispatch_layout(bool lk, bool rk, const CUtensorMap &tmL, const CUtensorMap &tmR, const KParams &kp, int grid,
-                    bool chained, cudaStream_t st) {
-  if (lk && rk) return launch_variant<BM, true, true, EngineT>(tmL, tmR, kp, grid, chained, st);
-  if (lk && !rk) return launch_variant<BM, true, false, EngineT>(tmL, tmR, kp, grid, chained, st);
-  if (!lk && rk) return launch_variant<BM, false, true, EngineT>(tmL, tmR, kp, grid, chained, st);
-  return launch_variant<BM, false, false, EngineT>(tmL, tmR, kp, grid, chained, st);
+                    bool alone, cudaStream_t st) {
+  if (lk && rk) return launch_variant<BM, true, true, EngineT>(tmL, tmR, kp, grid, alone, st);
+  if (lk && !rk) return launch_variant<BM, true, false, EngineT>(tmL, tmR, kp, grid, alone, st);
+  if (!lk && rk) return launch_variant<BM, false, true, EngineT>(tmL, tmR, kp, grid, alone, st);
+  return launch_variant<BM, false, false, EngineT>(tmL, tmR, kp, grid, alone, st);
 }
 
 // map_regular / map_balanced over `n` units into `P` blocks (the C restatement
@@ -913,17 +910,19 @@ int launch_trmm_fp64(const Fp64Launch &L, cudaStream_t stream, const char **why)
     grid = Q * CP;
   }
   const bool lk = L.lft_kmajor, rk = L.rgt_kmajor;
-  // Behind the lossless route: chained where every slot of the chip gets a CTA.
-  // Fewer are launched when the kernel in front is done: placed while it drains,
-  // two of them share an SM that is free first (3293 x 135: 6.6 ms, 3.98 so;
-  // where the route computes the call this costs 2 us, 5000 x 60 264 -> 266).
-  const bool chained = L.gate && grid >= L.num_sms * per_sm;
+  // Behind the lossless route the CTAs are placed while the kernel in front
+  // drains: where they do not fill every slot, two would share an SM that is free
+  // first (declined calls, ms: 3293 x 135, 156 tiles, 6.6, 3.96 so; 5000 x 60, 79
+  // tiles, 9.8 / 5.95; 2600 x 400, 287 tiles, 5.36 / 3.10).  They then ask for
+  // the shared memory of an SM alone and pull their tiles one by one.
+  const bool alone = L.gate && grid < L.num_sms * per_sm;
+  if (alone) grid = std::min(grid, L.num_sms);
   if (L.engine == UVATRMM_ENGINE_DMMA) {
-    if (BM == 128) return dispatch_layout<128, DmmaEngine>(lk, rk, tmL, tmR, kp, grid, chained, stream);
-    return dispatch_layout<64, DmmaEngine>(lk, rk, tmL, tmR, kp, grid, chained, stream);
+    if (BM == 128) return dispatch_layout<128, DmmaEngine>(lk, rk, tmL, tmR, kp, grid, alone, stream);
+    return dispatch_layout<64, DmmaEngine>(lk, rk, tmL, tmR, kp, grid, alone, stream);
   }
-  if (BM == 128) return dispatch_layout<128, DfmaEngine>(lk, rk, tmL, tmR, kp, grid, chained, stream);
-  return dispatch_layout<64, DfmaEngine>(lk, rk, tmL, tmR, kp, grid, chained, stream);
+  if (BM == 128) return dispatch_layout<128, DfmaEngine>(lk, rk, tmL, tmR, kp, grid, alone, stream);
+  return dispatch_layout<64, DfmaEngine>(lk, rk, tmL, tmR, kp, grid, alone, stream);
 }
 
 int fp64_group_prob(const Fp64Launch &L, int BM, Fp64GroupProb *out, const char **why) {
