@@ -426,8 +426,10 @@ int host_trmm(uvatrmm_handle_t h, int layout, int side, int uplo, int transa, in
   double *dB = static_cast<double *>(workspace(h, 1, (size_t)lb * t.n * 8));
   double *dC = static_cast<double *>(workspace(h, 2, (size_t)lb * t.n * 8));
   if (!dA || !dB || !dC) return tl_status;
-  cudaError_t e = copy_triangle_h2d(h, dA, la, A, lda, ka, t.uplo == CblasLower);
-  if (e == cudaSuccess) e = host_copy2d(h, dB, lb * 8, B, ldb * 8, t.m * 8, t.n, cudaMemcpyHostToDevice);
+  // (B first: its pages, which the caller has just written, are touched faster,
+  // and A's are touched while it moves.)
+  cudaError_t e = host_copy2d(h, dB, lb * 8, B, ldb * 8, t.m * 8, t.n, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = copy_triangle_h2d(h, dA, la, A, lda, ka, t.uplo == CblasLower);
   if (e != cudaSuccess) return drained(h, cuda_fail(e, "host to device copy"));
   const Route route = trmm_route(h, t, h->schedule, h->shape, false);
   const OzCtl *gate = nullptr;

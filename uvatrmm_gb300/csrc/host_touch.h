@@ -23,12 +23,15 @@ inline LinePart line_part(size_t width, size_t l, int tri) {
 template <class F>
 void for_each_page(uintptr_t base, size_t pitch, size_t width, size_t lines, int tri, size_t page, F &&f) {
   uintptr_t seen = base;  // no page below this one is left
-  for (size_t l = 0; l < lines; ++l) {
+  for (size_t l = 0; l < lines;) {
     const LinePart p = line_part(width, l, tri);
     const uintptr_t begin = base + l * pitch + p.lo, end = base + l * pitch + p.hi;
+    ++l;
     for (uintptr_t a = begin > seen ? begin : seen; a < end; a = seen) {
       f(a);
       seen = (a | (page - 1)) + 1;
+      const size_t next = (seen - base) / pitch;  // the lines before it lie below `seen`
+      if (next > l) l = next;
     }
   }
 }
