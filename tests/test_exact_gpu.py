@@ -3,8 +3,8 @@ cores, with every bit of every entry kept): each result is the exact product
 rounded once, so it equals the double-double oracle's rounding (cblas_dtrmm
 semantics, as the reference calls it at UVaTRMM/src/mm_triangular.c:374-387)
 entry by entry; operands it cannot hold go to the FP64 kernels, whose finite results are
-those of a handle pinned to the tile kernel, bit by bit (where the small
-kernel is not split along K; test_route_gpu.py has the split sizes)."""
+those of a handle pinned to the tile kernel, bit by bit."""
+# (Bit by bit where the small kernel is not split along K: test_route_gpu.py has the split sizes.)
 import numpy as np
 import pytest
 
