@@ -329,3 +329,34 @@ def test_declined_calls_take_little_longer_than_the_tile_kernel(built, side, ka,
         h.close()
         took.append(np.median(times[2:]))
     assert took[0] <= 1.3 * took[1], took
+
+
+@pytest.mark.parametrize("m,n,k", [(4, 87428, 452), (1, 37864, 4631), (3, 14222, 412), (2, 13501, 510)])
+def test_thin_gemms_are_not_slower_than_the_tile_kernel(built, m, n, k):
+    """GEMMs of a few rows and many columns, whose tiles cost what their rows do
+    (they took up to 70 % longer on the lossless route): at most 10 % over a
+    pinned handle, and right."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    A, B = (torch.rand(s, dtype=torch.float64, device="cuda", generator=gen) * 2 - 1 for s in ((k, m), (k, n)))
+    C = torch.zeros(n, m, dtype=torch.float64, device="cuda")  # column-major: C = A (m x k) * B (n x k)^T
+    took = []
+    for options in ({}, {"engine": u.ENGINE_DFMA}):
+        h = u.Handle(**options)
+        times = []
+        for _ in range(7):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            e0.record()
+            for _ in range(5):
+                h.dgemm_device(COL, NOTRANS, TRANS, m, n, k, 1.0, A, m, B, n, 0.0, C, m)
+            e1.record()
+            torch.cuda.synchronize()
+            times.append(e0.elapsed_time(e1))
+        if not options:
+            want = (A.t().double() @ B).t()
+            room = 8 * k * EPS * (A.t().abs() @ B.abs()).t()
+            assert bool(((C - want).abs() <= room).all())
+        h.close()
+        took.append(np.median(times[2:]))
+    assert took[0] <= 1.1 * took[1], took

@@ -197,7 +197,7 @@ inline int *scale_counters(uvatrmm_handle_t h) {
 // Kernel family for an M x N x K product (`tri`: one operand triangular) of
 // a single call on a handle whose options leave the choice open.
 enum class Route { kTile, kSmall, kExact };
-Route pick_route(int64_t M, int64_t N, int64_t K, bool tri, bool tri_left, bool in_place = false);
+Route pick_route(int64_t M, int64_t N, int64_t K, bool tri, bool tri_left, bool in_place = false, int64_t staged = 0);
 // Behind the lossless route of a TRMM: the small kernel instead of the tile
 // kernel where it is faster (the same bits where it is not split along K).
 bool small_behind_exact(int64_t M, int64_t N, int64_t K, bool tri_left);

@@ -67,7 +67,9 @@ int device_gemm(uvatrmm_handle_t h, int layout, int ta, int tb, int64_t m, int64
   const bool at = ta != CblasNoTrans, bt = tb != CblasNoTrans;
   int64_t ar = at ? k : m, ac = at ? m : k, br = bt ? n : k, bc = bt ? k : n;
   const bool free_choice = route_free(h, UVATRMM_SCHED_DYNAMIC, UVATRMM_SHAPE_TRAPEZOID);
-  const Route route = free_choice ? pick_route(m, n, k, false, true) : Route::kTile;
+  // (Of a thin GEMM the copy of a misaligned operand can be most of its time.)
+  const int64_t staged = m < 16 ? (tma_aligned(A, lda) ? 0 : 8 * m * k) + (tma_aligned(B, ldb) ? 0 : 8 * n * k) : 0;
+  const Route route = free_choice ? pick_route(m, n, k, false, true, false, staged) : Route::kTile;
   SmallProduct sp{};
   if (route == Route::kSmall) {
     sp.T = A;

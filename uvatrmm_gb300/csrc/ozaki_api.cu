@@ -255,6 +255,10 @@ namespace {
 constexpr int64_t kExactBytes = 16ll << 30;
 }
 
+namespace {
+bool thin_gemm(int64_t M, int64_t K, bool tri) { return !tri && M < 16 && K >= 64; }
+}  // namespace
+
 double tile_us(int64_t M, int64_t N, int64_t K, bool tri) {
   // An SM takes about 1 us per k of a 64 x 64 tile (2 FP64 FMAs per clock;
   // edge tiles by their 16-wide blocks), a little more for the one tile the
@@ -265,6 +269,15 @@ double tile_us(int64_t M, int64_t N, int64_t K, bool tri) {
   const double chain = 1.12 * k * (tri && K <= 64 ? 0.75 : 1.0);
   const double tiles = std::ceil(M / 64.0) * std::ceil(N / 64.0);
   const double work = tiles * (tri ? std::min(k, k / 2 + 15) : k) / 152;
+  // GEMMs of a few rows: rounds of two tiles per SM, whose rows go by twos (M x
+  // 50000 x 600, us: M = 2 380, 8 490, 12 730, 16 940, 64 3710), a last one of one
+  // per SM in half the time.
+  if (thin_gemm(M, K, tri)) {
+    const double full = std::floor(tiles / 304), last = tiles - 304 * full;
+    const double two = 0.034 * (double)((M + 1) / 2 * 2);
+    const double end = last > 152 ? std::max(0.21, two) : last > 0 ? std::max(0.21, two / 2) : 0.0;
+    return 9 + k * part(N) * (full * std::max(0.21, two) + end);
+  }
   return 9 + per_k * std::max(chain, 1.05 * work + 0.25 * k);
 }
 
@@ -273,12 +286,12 @@ double exact_us(int64_t M, int64_t N, int64_t K, bool tri) {
   // are one launch, which is left out: entries of wide spans need more moduli,
   // and would lose at 240 x 240 what others gain, 40 against 29 us); scaling and slicing per operand
   // entry (half of the K x K triangular operand); rounds of 256 x 256 residue
-  // tiles over the 76 SM pairs; product residues and reassembly.
+  // tiles over the 76 SM pairs; product residues and (of few rows: little) reassembly.
   const double m = (double)M, n = (double)N, k = (double)K;
   const double entries = k * (m + n) - (tri ? 0.5 * k * k : 0.0);
   const double pm = std::ceil(m / 256), pn = std::ceil(n / 256);
-  return 30 + 1.05e-5 * entries + std::ceil(pm * pn * 15 / 76) * (1.2 + 0.0062 * k * (tri ? 0.6 : 1.0)) +
-         1.2e-5 * pm * 256 * pn * 256;
+  const double rounds = std::ceil(pm * pn * 15 / 76) * (1.2 + 0.0062 * k * (tri ? 0.6 : 1.0));
+  return 30 + 1.05e-5 * entries + rounds + (thin_gemm(M, K, tri) ? 0.6e-5 : 1.2e-5) * pm * 256 * pn * 256;
 }
 
 // The fastest by the three estimates, which were fitted to (us, tile kernel /
@@ -290,10 +303,11 @@ double exact_us(int64_t M, int64_t N, int64_t K, bool tri) {
 //           1000 x 1000 2018 / 951 / 84   4000 x 1     1122 / 34 / 211
 // `in_place`: the tile kernel's copy of B counts as well (the small kernel
 // and the route need none); it does not move calls to or from the route.
-Route pick_route(int64_t M, int64_t N, int64_t K, bool tri, bool tri_left, bool in_place) {
+// `staged`: bytes of operands that only the tile kernel copies first.
+Route pick_route(int64_t M, int64_t N, int64_t K, bool tri, bool tri_left, bool in_place, int64_t staged) {
   const bool by_cols = !tri || tri_left;
   const double small = small_us(by_cols ? M : N, by_cols ? N : M, K, tri);
-  const double tile = tile_us(M, N, K, tri), exact = exact_us(M, N, K, tri);
+  const double tile = tile_us(M, N, K, tri) + staged / 0.85e6, exact = exact_us(M, N, K, tri);
   if (exact < std::min(small, tile)) return Route::kExact;
   const double copy = in_place ? 6 + 16.0 * M * N / 4e6 : 0.0;
   return small <= tile + copy ? Route::kSmall : Route::kTile;
